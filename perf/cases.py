@@ -10,6 +10,7 @@ call, work() the bytes and operations it cannot do without, exact() the outputs 
   rhs3d      the same on a periodic cube (3D Euler, plain flux divergence)
   igr        rhs! with the IGR source (a conjugate-gradient solve per evaluation)
   steps      solve() with SSP-RK3 and the HistoryCallback, host state in and out
+  advance    a few more steps of a host-held state (pinned arrays, in place)
   channel    solve() with inlet, outlet and slip walls (the reference's boundary set-up)
   ensemble   solve() over independent clouds of different sizes in one context
   gradient   d loss(u(T)) / d u0 through torch.autograd (record and reverse sweep)
@@ -44,8 +45,9 @@ def listed():
         dict(name="rhs_1m", kind="rhs", nx=1024, ny=1024, k=35, deg=3, visc="rv", hv=True, prec="fp64"),
         # time stepping of the vortex benchmark (262,144 nodes, residual viscosity)
         dict(name="steps_vortex", kind="steps", nx=512, ny=512, k=35, deg=3, hv=False, prec="fp64", nsteps=32),
-        # the FP32-apply form on the 1M problem
-        dict(name="steps_1m_fp32", kind="steps", nx=1024, ny=1024, k=35, deg=3, hv=True, prec="fp32", nsteps=24),
+        # the FP32-apply form on the 1M problem, a caller's loop that looks at the state
+        # every eight steps
+        dict(name="advance_1m_fp32", kind="advance", nx=1024, ny=1024, k=35, deg=3, hv=True, prec="fp32", nsteps=8),
         # the reference's boundary set-up: Dirichlet inlet (host callback), outlet, walls
         dict(name="channel", kind="channel", n=64, k=20, deg=3, nsteps=20),
         # 3D Euler on a cube of 64^3 nodes
@@ -68,7 +70,7 @@ def _log(rng, lo, hi):
 
 
 def draw(rng):
-    kind = rng.choice(["rhs", "rhs", "rhs", "steps", "steps", "channel", "rhs3d", "igr", "ensemble",
+    kind = rng.choice(["rhs", "rhs", "rhs", "steps", "advance", "channel", "rhs3d", "igr", "ensemble",
                        "gradient", "stencils", "weights"])
     k, deg = rng.choice([(35, 3), (35, 3), (28, 3), (24, 2), (20, 2)])
     if kind == "rhs":
@@ -79,6 +81,9 @@ def draw(rng):
         return dict(kind=kind, nx=_log(rng, 33, 900), ny=_log(rng, 33, 900), k=k, deg=deg,
                     hv=rng.random() < 0.5, prec=rng.choice(["fp64", "fp64", "fp32"]),
                     nsteps=rng.randint(4, 32))
+    if kind == "advance":
+        return dict(kind=kind, nx=_log(rng, 33, 1000), ny=_log(rng, 33, 1000), k=k, deg=deg,
+                    hv=rng.random() < 0.5, prec=rng.choice(["fp64", "fp32"]), nsteps=rng.randint(1, 8))
     if kind == "channel":
         return dict(kind=kind, n=_log(rng, 32, 250), k=rng.choice([20, 24, 35]), deg=3,
                     nsteps=rng.randint(4, 20))
@@ -155,12 +160,13 @@ def _channel(c, seed):
 
 
 def _channel_state(pts, seed):
-    """A uniform flow along x with a seeded smooth bump of density and pressure."""
+    """Flow along x with a transverse part that vanishes at the walls and a seeded smooth
+    bump of density and pressure."""
     g = np.random.default_rng(seed)
     cx, cy = g.uniform(0.35, 0.65, 2)
     b = 0.2 * np.exp(-((pts[:, 0] - cx) ** 2 + (pts[:, 1] - cy) ** 2) / 0.02)
-    rho, u, p = 1.0 + b, np.full(len(b), 0.4), 1.0 + b
-    return np.ascontiguousarray(np.stack([rho, rho * u, 0 * u, p / (GAMMA - 1.0) + 0.5 * rho * u * u]))
+    rho, u, v, p = 1.0 + b, np.full(len(b), 0.4), 0.1 * np.sin(np.pi * pts[:, 1]), 1.0 + b
+    return np.ascontiguousarray(np.stack([rho, rho * u, rho * v, p / (GAMMA - 1.0) + 0.5 * rho * (u * u + v * v)]))
 
 
 _INLET = np.array([1.0, 0.4, 0.0, 1.0 / (GAMMA - 1.0) + 0.5 * 0.16])
@@ -212,6 +218,12 @@ def prepare(case, seed):
         semi = _euler(c, pts, per, c["prec"], "rv", c["hv"])
         dt = 0.1 * h
         return dict(kind=kind, ode=M.ODEProblem(_waves(pts, per, seed), (0.0, c["nsteps"] * dt), semi), dt=dt)
+    if kind == "advance":
+        pts, per, h = _cloud(c, seed)
+        semi = _euler(c, pts, per, c["prec"], "rv", c["hv"])
+        semi.domain.ctx.history_init(3)
+        u = torch.from_numpy(_waves(pts, per, seed)).pin_memory()
+        return dict(kind=kind, semi=semi, u=u, t=0.0, dt=0.1 * h, nsteps=c["nsteps"])
     if kind == "channel":
         pts, bt, h = _channel(c, seed)
         solver = _solver(c)
@@ -266,6 +278,10 @@ def run(state):
     if kind == "steps":
         sol = M.solve(state["ode"], M.SSPRK33(), dt=state["dt"], callback=M.HistoryCallback(3))
         return sol.u, sol.t
+    if kind == "advance":
+        u = state["u"].numpy()
+        state["t"] = state["semi"].domain.ctx.ssprk33_host(u, state["t"], state["dt"], state["nsteps"])
+        return u
     if kind == "gradient":
         u0 = state["u0"].clone().requires_grad_(True)
         uT = autodiff.ssprk33_solve(u0, state["semi"], 0.0, state["dt"], state["nsteps"])
@@ -294,7 +310,7 @@ def work(case):
     per product of a weight with a flux or state (per system: the factorisation)."""
     c, kind = case, case["kind"]
     k = c.get("k", 0)
-    if kind in ("rhs", "steps", "channel", "ensemble", "igr", "gradient"):
+    if kind in ("rhs", "steps", "advance", "channel", "ensemble", "igr", "gradient"):
         s = 4 if c.get("prec") == "fp32" else 8
         if kind == "channel":
             n = c["n"] ** 2 + 4 * c["n"]
@@ -522,9 +538,9 @@ def exact(case, seed):
     c, kind = case, case["kind"]
     dev = _dev()
     up = lambda a: torch.from_numpy(a).to(dev)  # noqa: E731
-    if kind in ("rhs", "steps", "igr", "gradient"):
+    if kind in ("rhs", "steps", "advance", "igr", "gradient"):
         pts, per, h = _cloud(c, seed)
-        visc = "rv" if kind == "steps" else c.get("visc", "none")
+        visc = "rv" if kind in ("steps", "advance") else c.get("visc", "none")
         e = _Exact(pts, c["k"], c["deg"], per, (c["nx"], c["ny"]), visc, c.get("hv", False))
         u = up(_waves(pts, per, seed))
         if kind == "igr":
@@ -533,8 +549,9 @@ def exact(case, seed):
             e.approx_du, e.si = up(_approx_du(u.cpu().numpy())), 3
             return e.rhs(u)
         dt = 0.1 * h
-        if kind == "steps":
-            return e.solve(u, dt, c["nsteps"]).cpu(), c["nsteps"] * dt
+        if kind in ("steps", "advance"):
+            uT = e.solve(u, dt, c["nsteps"]).cpu()
+            return (uT, c["nsteps"] * dt) if kind == "steps" else uT
         u.requires_grad_(True)
         uT = e.solve(u, dt, c["nsteps"], history=False)
         (0.5 * (uT[0] - up(_waves(pts, per, seed + 1)[0])).square().sum()).backward()
