@@ -230,7 +230,7 @@ enum { MFT_OPT_GATHER = 0, MFT_OPT_TUNED_FWD = 1, MFT_OPT_TUNED_REV = 2,
        MFT_OPT_ENTRY_ORDER = 12, MFT_OPT_BANK_FWD = 13, MFT_OPT_BANK_REV = 14,
        MFT_OPT_FUSE_FLUX = 15, MFT_OPT_FLUX_FUSED = 16 };
 /* MFT_OPT_FUSE_FLUX (default 1): in the double-word form, when every row group is staged
- * and the forward gather's variant is 7, 11 or 12, that gather forms each staged
+ * and the forward gather's variant is 7, 9, 11 or 12, that gather forms each staged
  * neighbour's state and flux pairs from the FP64 state while staging, and the separate
  * flux kernel (which writes those pairs for every node) is skipped; 0 always runs it.  The
  * results are the same bits either way.  Read-only MFT_OPT_FLUX_FUSED: 1 when the last
@@ -264,7 +264,9 @@ enum { MFT_OPT_GATHER = 0, MFT_OPT_TUNED_FWD = 1, MFT_OPT_TUNED_REV = 2,
  * layout rows staged in shared memory by coalesced asynchronous copies and read from there (16-bit
  * positions instead of the 32-bit indices; a group with more than 640 distinct
  * neighbours gathers directly; registers capped at three blocks per SM), 8 = 7 capped at
- * four blocks per SM, 9 and 11 = staged with four and three entries per iteration, 10 = 7
+ * four blocks per SM, 9 = staged with the positions and weights of three entries loaded ahead
+ * while three accumulate (registers capped at two blocks per SM), 11 = staged with three
+ * entries per iteration, 10 = 7
  * with the streamed position and weight arrays prefetched into L2 as in 4, 12 = 7 with L2
  * eviction-priority hints (streamed arrays evict-first, the intermediates the transpose
  * gather reads back evict-last);

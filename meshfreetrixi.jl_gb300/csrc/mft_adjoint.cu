@@ -178,8 +178,8 @@ __global__ void k_lam_pairs(int64_t n, const double* __restrict__ lam, BcDev bc,
   if (BC) mask_rows<4>(bc, i, l);
   const float2 a = dw::split(l[0]), b = dw::split(l[1]), c = dw::split(l[2]),
                d = dw::split(l[3]);
-  out[i * 2] = make_float4(a.x, a.y, b.x, b.y);
-  out[i * 2 + 1] = make_float4(c.x, c.y, d.x, d.y);
+  out[i * 2] = dw::chunk(a, b);
+  out[i * 2 + 1] = dw::chunk(c, d);
 }
 
 // The adjoint gather of 2D Euler in double-word FP32 arithmetic (as the forward form's
@@ -190,11 +190,10 @@ __global__ void k_lam_pairs(int64_t n, const double* __restrict__ lam, BcDev bc,
 template <bool BC, int HV, bool HALO>
 __global__ void __launch_bounds__(HALO ? kHaloRows : kBlock) k_adj_dw(AdjArgs a) {
   const int64_t row = blockIdx.x * (int64_t)(HALO ? (int)blockDim.x : kBlock) + threadIdx.x;
-  const float* __restrict__ L = reinterpret_cast<const float*>(a.lamdw);
+  const float4* __restrict__ L4 = reinterpret_cast<const float4*>(a.lamdw);
   extern __shared__ float4 hsm[];
   bool staged = false;
   if (HALO) {
-    const float4* L4 = reinterpret_cast<const float4*>(a.lamdw);
     staged = stage_halo<2>(a.ell, hsm, [&](int k, int64_t c) { return L4 + c * 2 + k; });
   }
   if (row >= a.n) return;
@@ -202,32 +201,33 @@ __global__ void __launch_bounds__(HALO ? kHaloRows : kBlock) k_adj_dw(AdjArgs a)
   const int64_t base = a.ell.slice_off[row >> 5] + (row & 31);
   const int len = a.ell.row_len[row];
   const int hs = a.ell.halo_stride;
-  dw::Acc gx[4], gy[4], gh[4];
+  dw::Acc2 gx[2], gy[2], gh[2];
 #pragma unroll
-  for (int v = 0; v < 4; ++v) { gx[v] = dw::zero(); gy[v] = dw::zero(); gh[v] = dw::zero(); }
+  for (int k = 0; k < 2; ++k) gx[k] = gy[k] = gh[k] = dw::zero2();
 #pragma unroll 2
   for (int j = 0; j < len; ++j) {
     const int64_t p = base + ((int64_t)j << 5);
-    const float2 wx = __ldg(a.wdw[0] + p), wy = __ldg(a.wdw[1] + p);
-    F8 ll;
+    const float4 wxy = __ldg(a.wxydw + p);
+    dw::DW2 l[2];
     if (HALO && staged) {
       const int lc = __ldg(a.ell.lcol + p);
-      ll.lo = hsm[lc];
-      ll.hi = hsm[hs + lc];
+      l[0] = dw::pair2(hsm[halo_at<2>(0, lc, hs)]);
+      l[1] = dw::pair2(hsm[halo_at<2>(1, lc, hs)]);
     } else {
-      ll = ldg_f8(L + (int64_t)__ldg(a.ell.col + p) * 8);
+      const int64_t c = __ldg(a.ell.col + p);
+      l[0] = dw::pair2(__ldg(L4 + c * 2));
+      l[1] = dw::pair2(__ldg(L4 + c * 2 + 1));
     }
-    const float2 l[4] = {make_float2(ll.lo.x, ll.lo.y), make_float2(ll.lo.z, ll.lo.w),
-                         make_float2(ll.hi.x, ll.hi.y), make_float2(ll.hi.z, ll.hi.w)};
+    const dw::DW2 wx = dw::both(dw::chunk_a(wxy)), wy = dw::both(dw::chunk_b(wxy));
 #pragma unroll
-    for (int v = 0; v < 4; ++v) {
-      dw::fma_acc(gx[v], wx, l[v]);
-      dw::fma_acc(gy[v], wy, l[v]);
+    for (int k = 0; k < 2; ++k) {
+      dw::fma_acc2(gx[k], wx, l[k]);
+      dw::fma_acc2(gy[k], wy, l[k]);
     }
     if constexpr (HV == 2) {
-      const float2 wh = __ldg(a.whdw + p);
+      const dw::DW2 wh = dw::both(__ldg(a.whdw + p));
 #pragma unroll
-      for (int v = 0; v < 4; ++v) dw::fma_acc(gh[v], wh, l[v]);
+      for (int k = 0; k < 2; ++k) dw::fma_acc2(gh[k], wh, l[k]);
     }
   }
   // the Jacobian product in double-word arithmetic from the sums as pairs
@@ -235,9 +235,10 @@ __global__ void __launch_bounds__(HALO ? kHaloRows : kBlock) k_adj_dw(AdjArgs a)
   double ghd[4];
 #pragma unroll
   for (int v = 0; v < 4; ++v) {
-    gxp[v] = dw::to_pair(gx[v]);
-    gyp[v] = dw::to_pair(gy[v]);
-    ghd[v] = HV ? dw::to_double(gh[v]) : 0.0;
+    const int k = v >> 1;
+    gxp[v] = dw::to_pair(v & 1 ? dw::second(gx[k]) : dw::first(gx[k]));
+    gyp[v] = dw::to_pair(v & 1 ? dw::second(gy[k]) : dw::first(gy[k]));
+    ghd[v] = HV ? dw::to_double(v & 1 ? dw::second(gh[k]) : dw::first(gh[k])) : 0.0;
   }
   adj_finish<4, true, BC, HV>(a, i, nullptr, nullptr, ghd, gxp, gyp);
 }

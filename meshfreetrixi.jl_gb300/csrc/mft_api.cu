@@ -534,7 +534,7 @@ void ensure_work(mft_ctx* c) {
     c->tdw.alloc((size_t)n * 2 * V);
     c->qdw.alloc(nv);
   }
-  if (use_dw3(c)) c->Fdw.alloc((size_t)n * 12);  // the 12 distinct flux pairs of a node
+  if (use_dw3(c)) c->Fdw.alloc((size_t)n * 14);  // a node's flux record, seven chunks
   if (c->precision == MFT_PREC_FP32) {
     for (auto* b : {&c->U32[0], &c->U32[1], &c->U32[2], &c->U32[3]}) b->alloc(nv);
     c->du_p32.alloc(nv);
@@ -617,18 +617,23 @@ void ensure_device_ops(mft_ctx* c) {
     c->rw32[k].alloc(c->rev.n_elems);
     for (auto* b : {&c->fw[k], &c->rw[k]}) b->zero(s);
     for (auto* b : {&c->fw32[k], &c->rw32[k]}) b->zero(s);
-    if (dw) {
-      c->fwdw[k].alloc(c->fwd.n_elems);
-      c->rwdw[k].alloc(c->rev.n_elems);
+    // double-word values: D_x and D_y share slot 0 as chunks (w_x, w_y)
+    const bool chunked = dw && k < 2;
+    const int home = chunked ? 0 : k;
+    if (dw && home == k) {
+      c->fwdw[k].alloc((size_t)c->fwd.n_elems * (chunked ? 2 : 1));
+      c->rwdw[k].alloc((size_t)c->rev.n_elems * (chunked ? 2 : 1));
       for (auto* b : {&c->fwdw[k], &c->rwdw[k]}) b->zero(s);
     } else {
       c->fwdw[k].release();
       c->rwdw[k].release();
     }
-    launch_scatter_values((int64_t)v.size(), c->fwd_pos.p, d_v.p, c->fw[k].p, c->fw32[k].p,
-                          c->fwdw[k].p, s);
-    launch_scatter_values((int64_t)v.size(), c->rev_pos.p, d_v.p, c->rw[k].p, c->rw32[k].p,
-                          c->rwdw[k].p, s);
+    float2* fdw = dw ? c->fwdw[home].p : nullptr;
+    float2* rdw = dw ? c->rwdw[home].p : nullptr;
+    launch_scatter_values((int64_t)v.size(), c->fwd_pos.p, d_v.p, c->fw[k].p, c->fw32[k].p, fdw,
+                          chunked ? k : -1, s);
+    launch_scatter_values((int64_t)v.size(), c->rev_pos.p, d_v.p, c->rw[k].p, c->rw32[k].p, rdw,
+                          chunked ? k : -1, s);
   }
   MFT_CUDA(cudaStreamSynchronize(s));
   c->dev_dirty = false;
@@ -968,9 +973,10 @@ void eval_rhs(mft_ctx* c, double* us, float* us32, double t, const Epilogue& ep_
     fa.ep = ep;
     if (use_dw3(c)) {
       // double-word form: flux pairs per node, sums of double-word products
-      MFT_REQUIRE(c->Fdw.p && c->fwdw[0].p && c->fwdw[1].p && c->fwdw[2].p, MFT_ERR_STATE,
+      MFT_REQUIRE(c->Fdw.p && c->fwdw[0].p && c->fwdw[2].p, MFT_ERR_STATE,
                   "double-word 3D buffers not allocated");
-      for (int d = 0; d < 3; ++d) fa.wdw[d] = c->fwdw[d].p;
+      fa.wxydw = reinterpret_cast<const float4*>(c->fwdw[0].p);
+      fa.wzdw = c->fwdw[2].p;
       fa.Fdw = c->Fdw.p;
       {
         NvtxRange rng("calc fluxes");
@@ -1075,7 +1081,7 @@ void eval_rhs(mft_ctx* c, double* us, float* us32, double t, const Epilogue& ep_
   }
 
   // 2. flux per node (FP64 Euler; double-word pairs of the flux and the state for the
-  // double-word gathers).  The staged double-word forward variants 7, 11 and 12 can form
+  // double-word gathers).  The staged double-word forward variants 7, 9, 11 and 12 can form
   // those records while staging when every row group is staged; once such a variant is
   // the chosen one the flux kernel is skipped (it still runs in the evaluation that tunes,
   // whose unfused variants read its pairs).
@@ -1166,7 +1172,7 @@ void eval_rhs(mft_ctx* c, double* us, float* us32, double t, const Epilogue& ep_
     ea.ctr = c->d_ctr.p;
   }
   if (dw) {
-    for (int d = 0; d < 3; ++d) fa.wdw[d] = d < c->dim ? c->fwdw[d].p : nullptr;
+    fa.wxydw = reinterpret_cast<const float4*>(c->fwdw[0].p);
     fa.wldw = wl_slot >= 0 ? c->fwdw[wl_slot].p : nullptr;
     fa.Fdw = c->Fdw.p;
     fa.udw = c->udw.p;
@@ -1210,7 +1216,7 @@ void eval_rhs(mft_ctx* c, double* us, float* us32, double t, const Epilogue& ep_
   ra.s = c->t.p;
   ra.s32 = c->t32.p;
   if (dw) {
-    for (int d = 0; d < 3; ++d) ra.wdw[d] = d < c->dim ? c->rwdw[d].p : nullptr;
+    ra.wxydw = reinterpret_cast<const float4*>(c->rwdw[0].p);
     ra.wldw = tominec ? c->rwdw[kSlotLap].p : nullptr;
     ra.sdw = c->tdw.p;
     ra.qdw = c->qdw.p;
@@ -2694,8 +2700,7 @@ void eval_rhs_adjoint(mft_ctx* c, const double* u, const double* lam, int kind, 
   ProfScope ps(c, MFT_K_ADJ);
   if (use_dw(c) && hv != 1) {
     ensure_device_ops(c);
-    a.wdw[0] = c->rwdw[0].p;
-    a.wdw[1] = c->rwdw[1].p;
+    a.wxydw = reinterpret_cast<const float4*>(c->rwdw[0].p);
     a.whdw = hv == 2 ? c->rwdw[kSlotHv].p : nullptr;
     c->adj_lamdw.alloc((size_t)c->n * 4);
     // staged unless a fixed direct variant of the double-word gathers is requested

@@ -615,15 +615,10 @@ __global__ void __launch_bounds__(kBlock) k_eps(EpsArgs a) {
   }
   if (a.tdw) {
     // s = eps * t in double-word arithmetic (eps split once per node)
-    const float2 e2 = dw::split(eps);
+    const dw::DW2 e2 = dw::both(dw::split(eps));
     float4* t4 = reinterpret_cast<float4*>(a.tdw) + i * V;
 #pragma unroll
-    for (int q = 0; q < V; ++q) {
-      const float4 x = t4[q];
-      const float2 lo = dw::mul(e2, make_float2(x.x, x.y));
-      const float2 hi = dw::mul(e2, make_float2(x.z, x.w));
-      t4[q] = make_float4(lo.x, lo.y, hi.x, hi.y);
-    }
+    for (int q = 0; q < V; ++q) t4[q] = dw::chunk(dw::mul(e2, dw::pair2(t4[q])));
   }
   if (a.t32) {
     const float e32 = __double2float_rn(eps);
@@ -767,13 +762,22 @@ __global__ void k_differs(const double* __restrict__ a, const double* __restrict
 
 __global__ void k_scatter_values(int64_t nnz, const int64_t* __restrict__ pos,
                                  const double* __restrict__ v, double* __restrict__ out,
-                                 float* __restrict__ out32, float2* __restrict__ outdw) {
+                                 float* __restrict__ out32, float2* __restrict__ outdw,
+                                 int part) {
   const int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (e >= nnz) return;
   const int64_t p = pos[e];
   out[p] = v[e];
   if (out32) out32[p] = fpconv::d2f(v[e]);
-  if (outdw) outdw[p] = dw::split(v[e]);
+  if (!outdw) return;
+  const float2 w = dw::split(v[e]);
+  if (part < 0) {
+    outdw[p] = w;
+  } else {
+    float* o = reinterpret_cast<float*>(outdw) + p * 4 + part;
+    o[0] = w.x;
+    o[2] = w.y;
+  }
 }
 
 inline unsigned grid_for(int64_t n, int block) { return (unsigned)((n + block - 1) / block); }
@@ -783,9 +787,9 @@ inline unsigned grid_for(int64_t n, int block) { return (unsigned)((n + block - 
 // ====================================================================== launchers
 
 void launch_scatter_values(int64_t nnz, const int64_t* pos, const double* v, double* out,
-                           float* out32, float2* outdw, cudaStream_t s) {
+                           float* out32, float2* outdw, int part, cudaStream_t s) {
   if (nnz <= 0) return;
-  k_scatter_values<<<grid_for(nnz, 256), 256, 0, s>>>(nnz, pos, v, out, out32, outdw);
+  k_scatter_values<<<grid_for(nnz, 256), 256, 0, s>>>(nnz, pos, v, out, out32, outdw, part);
   MFT_LAUNCH_CHECK();
 }
 
@@ -929,6 +933,7 @@ void prepare_eps(EpsArgs& a) {
   a.rv_coef = (0.5 * a.c_rv) * (a.h * a.h);
   a.uw_bound = a.uw_coef * a.uw_coef * ((1.0 - 1e-12) / (1.0 + 1e-12));
   a.gg1 = a.gamma * (a.gamma - 1.0);
+  a.gg1_32 = (float)a.gg1;
   const float h32 = (float)a.h;
   a.gamma32 = (float)a.gamma;
   a.gm1_32 = (float)(a.gamma - 1.0);

@@ -21,6 +21,8 @@ namespace {
 
 using namespace dev;
 
+constexpr int kRec3 = 7;  // chunks of a node's double-word flux record
+
 inline unsigned grid_for(int64_t n, int block) { return (unsigned)((n + block - 1) / block); }
 
 // F[i] = (F_x, F_y, F_z), each the 5 components (rho v_d, rho v v_d + p e_d, (E + p) v_d):
@@ -92,13 +94,12 @@ __global__ void __launch_bounds__(kBlock) k_fwd3_f64(FwdArgs a) {
 
 // Double-word form: the state split into pairs and the flux formed in double-word
 // arithmetic (one reciprocal of rho refined by a Newton step).  The momentum flux is
-// symmetric, so the 15 flux components hold 12 distinct values, each formed once and
-// stored as one pair: F[i] = 6 float4 =
-//   (m1, m2), (m3, m1 v1 + p), (m2 v2 + p, m3 v3 + p), (m1 v2, m1 v3), (m2 v3, (E+p) v1),
-//   ((E+p) v2, (E+p) v3)
-// (96 bytes), and F_x = (m1, m1 v1 + p, m1 v2, m1 v3, (E+p) v1), F_y = (m2, m1 v2,
-// m2 v2 + p, m2 v3, (E+p) v2), F_z = (m3, m1 v3, m2 v3, m3 v3 + p, (E+p) v3).  The only
-// FP64 operations are the five splits.
+// symmetric, so the 15 flux components hold 12 distinct values, each formed once and stored
+// as the chunks of two that the gather multiplies (dw::chunk; xy = m1 m2 / rho and so on,
+// xx = m1 m1 / rho + p, ex = (E + p) v1):
+//   F[i] = (m1, ex), (m2, ey), (m3, ez), (xx, xy), (xy, yy), (xz, yz), (zz, zz)
+// (112 bytes), and F_x = (m1, xx, xy, xz, ex), F_y = (m2, xy, yy, yz, ey), F_z = (m3, xz, yz,
+// zz, ez).  The state is split on the integer pipe.
 __global__ void k_prep_euler3d_dw(int64_t n, float2 gm1, const double* __restrict__ u,
                                   float4* __restrict__ F) {
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -115,83 +116,99 @@ __global__ void k_prep_euler3d_dw(int64_t n, float2 gm1, const double* __restric
   const float2 zz = dw::add(dw::mul(m[2], v[2]), p);
   const float2 xy = dw::mul(m[0], v[1]), xz = dw::mul(m[0], v[2]), yz = dw::mul(m[1], v[2]);
   const float2 ex = dw::mul(ep, v[0]), ey = dw::mul(ep, v[1]), ez = dw::mul(ep, v[2]);
-  float4* Fi = F + i * 6;
-  Fi[0] = make_float4(m[0].x, m[0].y, m[1].x, m[1].y);
-  Fi[1] = make_float4(m[2].x, m[2].y, xx.x, xx.y);
-  Fi[2] = make_float4(yy.x, yy.y, zz.x, zz.y);
-  Fi[3] = make_float4(xy.x, xy.y, xz.x, xz.y);
-  Fi[4] = make_float4(yz.x, yz.y, ex.x, ex.y);
-  Fi[5] = make_float4(ey.x, ey.y, ez.x, ez.y);
+  float4* Fi = F + i * kRec3;
+  Fi[0] = dw::chunk(m[0], ex);
+  Fi[1] = dw::chunk(m[1], ey);
+  Fi[2] = dw::chunk(m[2], ez);
+  Fi[3] = dw::chunk(xx, xy);
+  Fi[4] = dw::chunk(xy, yy);
+  Fi[5] = dw::chunk(xz, yz);
+  Fi[6] = dw::chunk(zz, zz);
 }
 
-static __device__ __forceinline__ float2 lo2(float4 v) { return make_float2(v.x, v.y); }
-static __device__ __forceinline__ float2 hi2(float4 v) { return make_float2(v.z, v.w); }
+// Running sums of the 3D gather: (mass, energy), (momentum 1, 2), and momentum 3 in three
+// parts (x and y packed, z).
+struct Sums3 {
+  dw::Acc2 f04, f12, f3;
+  dw::Acc f3z;
+};
 
-// One stencil entry: the three weight pairs against the record's 15 flux components.
-static __device__ __forceinline__ void accum3(dw::Acc* f, const float2* w, const float4* q) {
-  const float2 m1 = lo2(q[0]), m2 = hi2(q[0]), m3 = lo2(q[1]), xx = hi2(q[1]);
-  const float2 yy = lo2(q[2]), zz = hi2(q[2]), xy = lo2(q[3]), xz = hi2(q[3]);
-  const float2 yz = lo2(q[4]), ex = hi2(q[4]), ey = lo2(q[5]), ez = hi2(q[5]);
-  const float2 fx[5] = {m1, xx, xy, xz, ex};
-  const float2 fy[5] = {m2, xy, yy, yz, ey};
-  const float2 fz[5] = {m3, xz, yz, zz, ez};
-#pragma unroll
-  for (int v = 0; v < 5; ++v) {
-    dw::fma_acc(f[v], w[0], fx[v]);
-    dw::fma_acc(f[v], w[1], fy[v]);
-    dw::fma_acc(f[v], w[2], fz[v]);
-  }
+// One stencil entry: the weights (wxy: the chunk of w_x and w_y) against the record's 15 flux
+// components, seven packed products and one scalar.
+static __device__ __forceinline__ void accum3(Sums3& s, float4 wxy, float2 wz, const float4* q) {
+  const dw::DW2 x = dw::both(dw::chunk_a(wxy)), y = dw::both(dw::chunk_b(wxy)), z = dw::both(wz);
+  const dw::DW2 xzyz = dw::pair2(q[5]);
+  dw::fma_acc2(s.f04, x, dw::pair2(q[0]));
+  dw::fma_acc2(s.f12, x, dw::pair2(q[3]));
+  dw::fma_acc2(s.f3, dw::pair2(wxy), xzyz);
+  dw::fma_acc2(s.f04, y, dw::pair2(q[1]));
+  dw::fma_acc2(s.f12, y, dw::pair2(q[4]));
+  dw::fma_acc(s.f3z, wz, dw::chunk_a(q[6]));
+  dw::fma_acc2(s.f04, z, dw::pair2(q[2]));
+  dw::fma_acc2(s.f12, z, xzyz);
 }
 
 // du_i = -sum_j (Dx_ij F_x + Dy_ij F_y + Dz_ij F_z)(node j) as compensated sums of
 // double-word products (mft_dw.cuh), the stage epilogue in FP64.  Per stencil entry: three
-// weight pairs and the neighbour's 96-byte flux record.  HALO: one block per row group
-// (ell.halo_rows rows) first stages the group's neighbour records in shared memory (six
+// weight pairs and the neighbour's 112-byte flux record.  HALO: one block per row group
+// (ell.halo_rows rows) first stages the group's neighbour records in shared memory (seven
 // 16-byte chunks each, mft_halo.cuh) and reads them from there; a group without a list
 // gathers directly.  Both read the same records in the same order: the same sums.
 template <bool HALO>
-__global__ void __launch_bounds__(HALO ? kHaloRows : kBlock) k_fwd3_dw(FwdArgs a) {
+__global__ void __launch_bounds__(HALO ? kHaloRows : kBlock, 2) k_fwd3_dw(FwdArgs a) {
   const int64_t r = blockIdx.x * (int64_t)(HALO ? (int)blockDim.x : kBlock) + threadIdx.x;
   const float4* __restrict__ F4 = reinterpret_cast<const float4*>(a.Fdw);
   extern __shared__ float4 hsm3[];
   bool staged = false;
-  if (HALO) staged = stage_halo<6>(a.ell, hsm3, [&](int k, int64_t c) { return F4 + c * 6 + k; });
+  if (HALO) staged = stage_halo<kRec3>(a.ell, hsm3, [&](int k, int64_t c) { return F4 + c * kRec3 + k; });
   if (r >= a.n) return;
   const int64_t i = ell_node(a.ell, r);
   const int64_t base = a.ell.slice_off[r >> 5] + (r & 31);
   const int len = a.ell.row_len[r];
   const int hs = a.ell.halo_stride;
-  dw::Acc f[5];
-#pragma unroll
-  for (int v = 0; v < 5; ++v) f[v] = dw::zero();
+  Sums3 f;
+  f.f04 = f.f12 = f.f3 = dw::zero2();
+  f.f3z = dw::zero();
   if (HALO && staged) {
-    const uint16_t* __restrict__ lcol = a.ell.lcol;
-#pragma unroll 2
-    for (int j = 0; j < len; ++j) {
-      const int64_t p = base + ((int64_t)j << 5);
-      const int lc = __ldg(lcol + p);
-      const float2 w[3] = {__ldg(a.wdw[0] + p), __ldg(a.wdw[1] + p), __ldg(a.wdw[2] + p)};
-      float4 q[6];
+    struct Streamed {
+      int lc;
+      float4 wxy;
+      float2 wz;
+    };
+    pipelined_row<4, Streamed>(
+        len,
+        [&](Streamed& e, int j) {
+          e.lc = __ldg(a.ell.lcol + base + j * 32);
+          e.wxy = __ldg(a.wxydw + base + j * 32);
+          e.wz = __ldg(a.wzdw + base + j * 32);
+        },
+        [&](const Streamed& e) {
+          float4 q[kRec3];
 #pragma unroll
-      for (int k = 0; k < 6; ++k) q[k] = hsm3[k * hs + lc];
-      accum3(f, w, q);
-    }
+          for (int k = 0; k < kRec3; ++k) q[k] = hsm3[halo_at<kRec3>(k, e.lc, hs)];
+          accum3(f, e.wxy, e.wz, q);
+        });
   } else {
     const int32_t* __restrict__ col = a.ell.col;
 #pragma unroll 2
     for (int j = 0; j < len; ++j) {
       const int64_t p = base + ((int64_t)j << 5);
       const int64_t c = __ldg(col + p);
-      const float2 w[3] = {__ldg(a.wdw[0] + p), __ldg(a.wdw[1] + p), __ldg(a.wdw[2] + p)};
-      float4 q[6];
+      const float4 wxy = __ldg(a.wxydw + p);
+      const float2 wz = __ldg(a.wzdw + p);
+      float4 q[kRec3];
 #pragma unroll
-      for (int k = 0; k < 6; ++k) q[k] = __ldg(F4 + c * 6 + k);
-      accum3(f, w, q);
+      for (int k = 0; k < kRec3; ++k) q[k] = __ldg(F4 + c * kRec3 + k);
+      accum3(f, wxy, wz, q);
     }
   }
   double du[5];
-#pragma unroll
-  for (int v = 0; v < 5; ++v) du[v] = -dw::to_double(f[v]);
+  du[0] = -dw::to_double(dw::first(f.f04));
+  du[1] = -dw::to_double(dw::first(f.f12));
+  du[2] = -dw::to_double(dw::second(f.f12));
+  du[3] = -dw::value(dw::add(dw::add(dw::to_pair(dw::first(f.f3)), dw::to_pair(dw::second(f.f3))),
+                             dw::to_pair(f.f3z)));
+  du[4] = -dw::to_double(dw::second(f.f04));
   finish_node<5>(a.ep, i, du);
 }
 
@@ -209,12 +226,12 @@ void launch_prep_euler3d_dw(int64_t n, double gamma, const double* u, float2* F,
 
 void launch_fwd3_dw(const FwdArgs& a, cudaStream_t s) {
   if (a.n <= 0) return;
-  MFT_REQUIRE(a.V == 5 && a.Fdw && a.wdw[0] && a.wdw[1] && a.wdw[2] && a.final_epilogue,
+  MFT_REQUIRE(a.V == 5 && a.Fdw && a.wxydw && a.wzdw && a.final_epilogue,
               MFT_ERR_STATE, "double-word 3D gather: arguments not set");
   if (a.ell.halo_off && a.ell.halo_rows > 0) {
-    // one block per row group, six chunks of the longest list in dynamic shared memory
+    // one block per row group, seven chunks of the longest list in dynamic shared memory
     // (above 48 KB a per-kernel opt-in, made once per device)
-    const size_t smem = (size_t)6 * a.ell.halo_stride * sizeof(float4);
+    const size_t smem = (size_t)kRec3 * a.ell.halo_stride * sizeof(float4);
     if (smem > 48 * 1024) {
       static std::mutex mu;
       static std::set<int> done;
@@ -223,7 +240,7 @@ void launch_fwd3_dw(const FwdArgs& a, cudaStream_t s) {
       std::lock_guard<std::mutex> lock(mu);
       if (done.insert(dev).second)
         MFT_CUDA(cudaFuncSetAttribute(k_fwd3_dw<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)(6 * kHaloMax * sizeof(float4))));
+                                      (int)(kRec3 * kHaloMax * sizeof(float4))));
     }
     const int rows = a.ell.halo_rows;
     k_fwd3_dw<true><<<grid_for(a.n, rows), rows, smem, s>>>(a);

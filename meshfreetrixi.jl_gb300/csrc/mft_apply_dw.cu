@@ -30,8 +30,6 @@ using namespace dev;
 
 inline unsigned grid_for(int64_t n, int block) { return (unsigned)((n + block - 1) / block); }
 
-static __device__ __forceinline__ float2 lo2(float4 v) { return make_float2(v.x, v.y); }
-
 // The streamed arrays of a warp's slice (column indices and up to three weight arrays,
 // read once per launch) requested into L2 a chunk of kPfSlots slots at a time by one
 // lane, ahead of the slots the warp gathers (the weights otherwise arrive from DRAM on
@@ -53,15 +51,14 @@ static __device__ __forceinline__ void prefetch_chunk(const SliceArrays& sa, int
       tma::bulk_prefetch_l2(static_cast<const char*>(sa.arr[k]) + e0 * sa.esize[k],
                             (uint32_t)(ne * sa.esize[k]));
 }
-static __device__ __forceinline__ float2 hi2(float4 v) { return make_float2(v.z, v.w); }
-
 
 // Per node: the state as double-word pairs and the Euler flux pair evaluated from them in
 // double-word arithmetic (the textbook flux, one reciprocal for both velocities; each
 // operation is accurate to about 2 u^2 of its operands, u = 2^-24), as the records the
-// forward gather reads: F = (Fx_0..3, Fy_0..3) in four float4 (Fx_0 = m1, Fy_0 = m2),
-// U = (u_0..3) in two, 8 floats per 4 values.  gm1 = gamma - 1 as a pair.  The only FP64
-// operations are the four splits of the state.  Shared by the flux kernel and the staged
+// forward gather reads, in chunks of two values (dw::chunk): U = (rho, m1), (m2, E) and
+// F = (fx1, f12), (f12, fy2), (fx3, fy3), (m1, m2), with f12 = m1 m2 / rho the x flux of m2
+// and the y flux of m1; the mass fluxes are m1 and m2.  gm1 = gamma - 1 as a pair.  The only
+// FP64 operations are the four splits of the state.  Shared by the flux kernel and the staged
 // gathers that form the records while staging, so both give the same bits.
 static __device__ __forceinline__ void euler_records(double2 a, double2 b, float2 gm1,
                                                      float4* F, float4* U) {
@@ -72,14 +69,14 @@ static __device__ __forceinline__ void euler_records(double2 a, double2 b, float
   const float2 a1 = dw::mul(m1, v1), a2 = dw::mul(m2, v2);
   const float2 p = dw::mul(gm1, dw::add(en, dw::neg(dw::scale2(dw::add(a1, a2), 0.5f))));
   const float2 ep = dw::add(en, p);
-  const float2 fx1 = dw::add(a1, p), fx2 = dw::mul(m1, v2), fx3 = dw::mul(ep, v1);
-  const float2 fy1 = dw::mul(m2, v1), fy2 = dw::add(a2, p), fy3 = dw::mul(ep, v2);
-  F[0] = make_float4(m1.x, m1.y, fx1.x, fx1.y);
-  F[1] = make_float4(fx2.x, fx2.y, fx3.x, fx3.y);
-  F[2] = make_float4(m2.x, m2.y, fy1.x, fy1.y);
-  F[3] = make_float4(fy2.x, fy2.y, fy3.x, fy3.y);
-  U[0] = make_float4(rho.x, rho.y, m1.x, m1.y);
-  U[1] = make_float4(m2.x, m2.y, en.x, en.y);
+  const float2 fx1 = dw::add(a1, p), f12 = dw::mul(m1, v2), fx3 = dw::mul(ep, v1);
+  const float2 fy2 = dw::add(a2, p), fy3 = dw::mul(ep, v2);
+  F[0] = dw::chunk(fx1, f12);
+  F[1] = dw::chunk(f12, fy2);
+  F[2] = dw::chunk(fx3, fy3);
+  F[3] = dw::chunk(m1, m2);
+  U[0] = dw::chunk(rho, m1);
+  U[1] = dw::chunk(m2, en);
 }
 
 __global__ void k_prep_euler_dw(int64_t n, float2 gm1, const double* __restrict__ u,
@@ -96,11 +93,17 @@ __global__ void k_prep_euler_dw(int64_t n, float2 gm1, const double* __restrict_
   U[i * 2 + 1] = uu[1];
 }
 
+// Chunks of a staged forward record: with the state needed (t, q or the Flyer term) the
+// three flux chunks and the two state chunks, whose m1 and m2 serve the mass flux too; else
+// the four flux chunks.
+template <bool NEEDU>
+constexpr int kFwdChunks = NEEDU ? 5 : 4;
+
 // Staging with the records formed on the fly: each thread reads the FP64 states of list
 // entries q and q + blockDim.x (both loads in flight together), forms their records
-// (euler_records) and writes the NCH chunks of each into shared memory at k * stride + q,
-// the layout stage_halo's copies give.  Returns false for a group without a list.
-template <int NCH>
+// (euler_records) and writes their chunks into shared memory where stage_halo's copies would
+// (halo_at).  Returns false for a group without a list.
+template <bool NEEDU>
 static __device__ __forceinline__ bool stage_halo_records(const EllView& ell, float4* sm,
                                                           const double* __restrict__ u,
                                                           float2 gm1) {
@@ -109,91 +112,127 @@ static __device__ __forceinline__ bool stage_halo_records(const EllView& ell, fl
   if (nh <= 0) return false;  // block-uniform
   const int hs = ell.halo_stride;
   const double2* __restrict__ u2 = reinterpret_cast<const double2*>(u);
+  auto put = [&](int q, double2 a, double2 b) {
+    float4 F[4], U[2];
+    euler_records(a, b, gm1, F, U);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) sm[halo_at<kFwdChunks<NEEDU>>(k, q, hs)] = F[k];
+    if (NEEDU) {
+      sm[halo_at<5>(3, q, hs)] = U[0];
+      sm[halo_at<5>(4, q, hs)] = U[1];
+    } else {
+      sm[halo_at<4>(3, q, hs)] = F[3];
+    }
+  };
   for (int q0 = threadIdx.x; q0 < nh; q0 += 2 * blockDim.x) {
     const int q1 = q0 + blockDim.x;
     const int64_t c0 = __ldg(ell.halo_col + h0 + q0);
     const int64_t c1 = q1 < nh ? (int64_t)__ldg(ell.halo_col + h0 + q1) : c0;
     const double2 a0 = __ldg(u2 + c0 * 2), b0 = __ldg(u2 + c0 * 2 + 1);
     const double2 a1 = __ldg(u2 + c1 * 2), b1 = __ldg(u2 + c1 * 2 + 1);
-    float4 rec[6];
-    euler_records(a0, b0, gm1, rec, rec + 4);
-#pragma unroll
-    for (int k = 0; k < NCH; ++k) sm[k * hs + q0] = rec[k];
-    if (q1 < nh) {
-      euler_records(a1, b1, gm1, rec, rec + 4);
-#pragma unroll
-      for (int k = 0; k < NCH; ++k) sm[k * hs + q1] = rec[k];
-    }
+    put(q0, a0, b0);
+    if (q1 < nh) put(q1, a1, b1);
   }
   __syncthreads();
   return true;
 }
 
-// One stencil entry of the forward gather: weights and the neighbour's flux and state
-// records, requested together.
+// One stencil entry of the forward gather: the weight pairs (wxy: the chunk of w_x and w_y)
+// and the neighbour's flux and state chunks, requested together.  f[3] = (m1, m2) only
+// without the state chunks.
 struct FwdEntry {
-  float2 wx, wy, wl;
-  F8 fa, fb, uu;
+  float4 wxy;
+  float2 wl;
+  float4 f[4], u[2];
 };
 
-template <bool WT, bool WQ, int FLY>
-static __device__ __forceinline__ FwdEntry fwd_load(const FwdArgs& a, const float* F,
-                                                    const float* U, int64_t p, int64_t c) {
+template <bool NEEDU, bool NEEDL>
+static __device__ __forceinline__ FwdEntry fwd_load(const FwdArgs& a, const float4* F,
+                                                    const float4* U, int64_t p, int64_t c) {
   FwdEntry e;
-  e.wx = __ldg(a.wdw[0] + p);
-  e.wy = __ldg(a.wdw[1] + p);
-  e.fa = ldg_f8(F + c * 16);
-  e.fb = ldg_f8(F + c * 16 + 8);
-  if (WT || WQ || FLY) e.uu = ldg_f8(U + c * 8);
-  if (WQ || FLY) e.wl = __ldg(a.wldw + p);
+  e.wxy = __ldg(a.wxydw + p);
+#pragma unroll
+  for (int k = 0; k < (NEEDU ? 3 : 4); ++k) e.f[k] = __ldg(F + c * 4 + k);
+  if (NEEDU) {
+    e.u[0] = __ldg(U + c * 2);
+    e.u[1] = __ldg(U + c * 2 + 1);
+  }
+  if (NEEDL) e.wl = __ldg(a.wldw + p);
   return e;
 }
 
-// The same entry with the neighbour's records read from the staged halo (lc: position
-// of the neighbour in the group's list).
-template <bool WT, bool WQ, int FLY, bool HINT = false>
-static __device__ __forceinline__ FwdEntry fwd_load_halo(const FwdArgs& a, const float4* sm,
-                                                         int hs, int64_t p, int lc,
-                                                         uint64_t pol = 0) {
+// The streamed arrays of a row in the staged loop: the row's element of slot j is element
+// 32 j of each.
+struct RowStream {
+  const uint16_t* lc;
+  const float4* wxy;
+  const float2* wl;
+};
+
+constexpr int kPipelined = 10;  // PIPE: pipelined_row
+
+// The streamed part of entry j of the row.
+struct Streamed {
+  int lc;
+  float4 wxy;
+  float2 wl;
+};
+template <bool XY, bool L, bool HINT = false>
+static __device__ __forceinline__ void stream_load(Streamed& e, const RowStream& w, int j,
+                                                   uint64_t pol = 0) {
+  const int o = j * 32;
+  e.lc = HINT ? ldg_hint(w.lc + o, pol) : __ldg(w.lc + o);
+  if (XY) e.wxy = HINT ? ldg_hint(w.wxy + o, pol) : __ldg(w.wxy + o);
+  if (L) e.wl = HINT ? ldg_hint(w.wl + o, pol) : __ldg(w.wl + o);
+}
+
+// The entry with the neighbour's records read from the staged halo.
+template <bool NEEDU, bool NEEDL>
+static __device__ __forceinline__ FwdEntry fwd_load_halo(const Streamed& x, const float4* sm,
+                                                         int hs) {
   FwdEntry e;
-  e.wx = HINT ? ldg_hint(a.wdw[0] + p, pol) : __ldg(a.wdw[0] + p);
-  e.wy = HINT ? ldg_hint(a.wdw[1] + p, pol) : __ldg(a.wdw[1] + p);
-  e.fa.lo = sm[lc];
-  e.fa.hi = sm[hs + lc];
-  e.fb.lo = sm[2 * hs + lc];
-  e.fb.hi = sm[3 * hs + lc];
-  if (WT || WQ || FLY) {
-    e.uu.lo = sm[4 * hs + lc];
-    e.uu.hi = sm[5 * hs + lc];
+  e.wxy = x.wxy;
+  if (NEEDL) e.wl = x.wl;
+  constexpr int N = kFwdChunks<NEEDU>;
+#pragma unroll
+  for (int k = 0; k < (NEEDU ? 3 : 4); ++k) e.f[k] = sm[halo_at<N>(k, x.lc, hs)];
+  if (NEEDU) {
+    e.u[0] = sm[halo_at<N>(3, x.lc, hs)];
+    e.u[1] = sm[halo_at<N>(4, x.lc, hs)];
   }
-  if (WQ || FLY) e.wl = HINT ? ldg_hint(a.wldw + p, pol) : __ldg(a.wldw + p);
   return e;
 }
 
-template <bool WT, bool WQ, int FLY>
-static __device__ __forceinline__ void fwd_accum(const FwdEntry& e, dw::Acc* f, dw::Acc* tx,
-                                                 dw::Acc* ty, dw::Acc* q) {
-  const float2 Fx[4] = {lo2(e.fa.lo), hi2(e.fa.lo), lo2(e.fa.hi), hi2(e.fa.hi)};
-  const float2 Fy[4] = {lo2(e.fb.lo), hi2(e.fb.lo), lo2(e.fb.hi), hi2(e.fb.hi)};
+// The forward gather's running sums, two values each: f12 = (momentum rows), f3 = (x part,
+// y part) of the energy row, f0 the same of the mass row (where t does not give it), and
+// t = (Dx u, Dy u), q over the four variables.
+struct FwdSums {
+  dw::Acc2 f0, f12, f3, tx[2], ty[2], q[2];
+};
+
+template <bool WT, bool NEEDL>
+static __device__ __forceinline__ void fwd_accum(const FwdEntry& e, FwdSums& s) {
+  constexpr bool NEEDU = WT || NEEDL;
+  const dw::DW2 wxy = dw::pair2(e.wxy);
+  const dw::DW2 wx = dw::both(dw::chunk_a(e.wxy)), wy = dw::both(dw::chunk_b(e.wxy));
+  dw::fma_acc2(s.f12, wx, dw::pair2(e.f[0]));
+  dw::fma_acc2(s.f12, wy, dw::pair2(e.f[1]));
+  dw::fma_acc2(s.f3, wxy, dw::pair2(e.f[2]));
+  // with t formed, the rho row is tx_1 + ty_2
+  if (!WT)
+    dw::fma_acc2(s.f0, wxy,
+                 NEEDU ? dw::pair2(dw::chunk_b(e.u[0]), dw::chunk_a(e.u[1])) : dw::pair2(e.f[3]));
+  if (WT) {
 #pragma unroll
-  for (int v = WT ? 1 : 0; v < 4; ++v) {
-    // Fx[0] = m1, Fy[0] = m2: with t formed, the rho row is tx1 + ty2
-    dw::fma_acc(f[v], e.wx, Fx[v]);
-    dw::fma_acc(f[v], e.wy, Fy[v]);
+    for (int k = 0; k < 2; ++k) {
+      dw::fma_acc2(s.tx[k], wx, dw::pair2(e.u[k]));
+      dw::fma_acc2(s.ty[k], wy, dw::pair2(e.u[k]));
+    }
   }
-  if (WT || WQ || FLY) {
-    const float2 uc[4] = {lo2(e.uu.lo), hi2(e.uu.lo), lo2(e.uu.hi), hi2(e.uu.hi)};
-    if (WT) {
+  if (NEEDL) {
+    const dw::DW2 wl = dw::both(e.wl);
 #pragma unroll
-      for (int v = 0; v < 4; ++v) {
-        dw::fma_acc(tx[v], e.wx, uc[v]);
-        dw::fma_acc(ty[v], e.wy, uc[v]);
-      }
-    }
-    if (WQ || FLY) {
-#pragma unroll
-      for (int v = 0; v < 4; ++v) dw::fma_acc(q[v], e.wl, uc[v]);
-    }
+    for (int k = 0; k < 2; ++k) dw::fma_acc2(s.q[k], wl, dw::pair2(e.u[k]));
   }
 }
 
@@ -209,7 +248,7 @@ static __device__ __forceinline__ void fwd_accum(const FwdEntry& e, dw::Acc* f, 
 // The variants form the same sums in the same order; the autotuner picks one.
 // HALO: blocks of one row group (ell.halo_rows rows) first stage the group's neighbour
 // records in shared memory and read them from there (groups without a list gather
-// directly); PIPE 0 or 2 then sets the loop's unrolling.  HINT: the staged loop reads the
+// directly); PIPE then sets the loop's unrolling, or kPipelined.  HINT: the staged loop reads the
 // streamed positions and weights with an L2 evict-first policy and the epilogue writes t,
 // q and the partial du with evict-last, which the transpose gather reads next.  FUSE: the
 // staged records are formed from the FP64 state while staging (stage_halo_records), so
@@ -219,33 +258,31 @@ template <bool WT, bool WQ, int FLY, int PIPE, int MINB, bool PREF, bool HALO, b
           bool FUSE = false>
 __global__ void __launch_bounds__(HALO ? kHaloRows : kBlock, MINB) k_fwd_euler_dw(FwdArgs a) {
   const int64_t r = blockIdx.x * (int64_t)(HALO ? (int)blockDim.x : kBlock) + threadIdx.x;
-  const float* __restrict__ F = reinterpret_cast<const float*>(a.Fdw);
-  const float* __restrict__ U = reinterpret_cast<const float*>(a.udw);
+  constexpr bool NEEDL = WQ || FLY != 0, NEEDU = WT || NEEDL;
+  const float4* __restrict__ F = reinterpret_cast<const float4*>(a.Fdw);
+  const float4* __restrict__ U = reinterpret_cast<const float4*>(a.udw);
   extern __shared__ float4 hsm[];
   bool staged = false;
-  constexpr int kNch = (WT || WQ || FLY) ? 6 : 4;
   if (HALO && FUSE) {
-    staged = stage_halo_records<kNch>(a.ell, hsm, a.ustate, a.gm1dw);
+    staged = stage_halo_records<NEEDU>(a.ell, hsm, a.ustate, a.gm1dw);
     if (!staged) {
       if (threadIdx.x == 0) atomicExch(a.err, MFT_ERR_STATE);
       return;
     }
   } else if (HALO) {
-    const float4* F4 = reinterpret_cast<const float4*>(a.Fdw);
-    const float4* U4 = reinterpret_cast<const float4*>(a.udw);
-    staged = stage_halo<kNch>(
-        a.ell, hsm, [&](int k, int64_t c) { return k < 4 ? F4 + c * 4 + k : U4 + c * 2 + (k - 4); });
+    staged = stage_halo<kFwdChunks<NEEDU>>(a.ell, hsm, [&](int k, int64_t c) {
+      return !NEEDU || k < 3 ? F + c * 4 + k : U + c * 2 + (k - 3);
+    });
   }
   if (r >= a.n) return;
   const int64_t i = ell_node(a.ell, r);
   const int64_t base = a.ell.slice_off[r >> 5] + (r & 31);
   const int len = a.ell.row_len[r];
   const int32_t* __restrict__ col = a.ell.col;
-  dw::Acc f[4], tx[4], ty[4], q[4];
+  FwdSums sum;
+  sum.f0 = sum.f12 = sum.f3 = dw::zero2();
 #pragma unroll
-  for (int v = 0; v < 4; ++v) {
-    f[v] = dw::zero(); tx[v] = dw::zero(); ty[v] = dw::zero(); q[v] = dw::zero();
-  }
+  for (int k = 0; k < 2; ++k) sum.tx[k] = sum.ty[k] = sum.q[k] = dw::zero2();
   const uint16_t* __restrict__ lcol = a.ell.lcol;
   const int hs = a.ell.halo_stride;
   if (HALO && staged) {
@@ -254,30 +291,51 @@ __global__ void __launch_bounds__(HALO ? kHaloRows : kBlock, MINB) k_fwd_euler_d
     const bool pf_lane = PREF && (threadIdx.x & 31) == 0;
     if (pf_lane) {
       sa.arr[0] = lcol; sa.esize[0] = 2;
-      sa.arr[1] = a.wdw[0]; sa.esize[1] = 8;
-      sa.arr[2] = a.wdw[1]; sa.esize[2] = 8;
-      sa.arr[3] = a.wldw; sa.esize[3] = 8;
-      sa.narr = (WQ || FLY) ? 4 : 3;
+      sa.arr[1] = a.wxydw; sa.esize[1] = 16;
+      sa.arr[2] = a.wldw; sa.esize[2] = 8;
+      sa.narr = NEEDL ? 3 : 2;
       s_lo = a.ell.slice_off[r >> 5];
       s_hi = a.ell.slice_off[(r >> 5) + 1];
       prefetch_chunk(sa, s_lo, s_hi, 0);
       prefetch_chunk(sa, s_lo, s_hi, 1);
     }
-    constexpr int UNR = PIPE < 1 ? 1 : PIPE;
+    constexpr int UNR = PIPE < 1 || PIPE == kPipelined ? 1 : PIPE;
     const uint64_t pol = HINT ? l2_evict_first() : 0;
-#pragma unroll UNR
-    for (int j = 0; j < len; ++j) {
-      if (pf_lane && (j % kPfSlots) == 0) prefetch_chunk(sa, s_lo, s_hi, j / kPfSlots + 2);
-      const int64_t p = base + ((int64_t)j << 5);
-      const int lc = HINT ? ldg_hint(lcol + p, pol) : __ldg(lcol + p);
-      fwd_accum<WT, WQ, FLY>(fwd_load_halo<WT, WQ, FLY, HINT>(a, hsm, hs, p, lc, pol), f, tx, ty, q);
+    RowStream w{lcol + base, a.wxydw + base, a.wldw + base};
+    auto load = [&](Streamed& x, int j) { stream_load<true, NEEDL, HINT>(x, w, j, pol); };
+    auto use = [&](const Streamed& x) {
+      fwd_accum<WT, NEEDL>(fwd_load_halo<NEEDU, NEEDL>(x, hsm, hs), sum);
+    };
+    if constexpr (PIPE == kPipelined) {
+      pipelined_row<3, Streamed>(len, load, use);
+    } else {
+      int j = 0;
+      for (; j + UNR <= len; j += UNR) {
+        if (pf_lane && (j % kPfSlots) < UNR) prefetch_chunk(sa, s_lo, s_hi, j / kPfSlots + 2);
+        Streamed x[UNR];
+#pragma unroll
+        for (int k = 0; k < UNR; ++k) load(x[k], k);
+#pragma unroll
+        for (int k = 0; k < UNR; ++k) use(x[k]);
+        w.lc += UNR * 32;
+        w.wxy += UNR * 32;
+        w.wl += UNR * 32;
+      }
+      for (; j < len; ++j) {
+        Streamed x;
+        load(x, 0);
+        use(x);
+        w.lc += 32;
+        w.wxy += 32;
+        w.wl += 32;
+      }
     }
   } else if (PIPE == 0) {
 #pragma unroll 1
     for (int j = 0; j < len; ++j) {
       const int64_t p = base + ((int64_t)j << 5);
       const int64_t c = __ldg(col + p);
-      fwd_accum<WT, WQ, FLY>(fwd_load<WT, WQ, FLY>(a, F, U, p, c), f, tx, ty, q);
+      fwd_accum<WT, NEEDL>(fwd_load<NEEDU, NEEDL>(a, F, U, p, c), sum);
     }
   } else if (PIPE == 2 || (HALO && PIPE > 2)) {
     SliceArrays sa{};
@@ -285,10 +343,9 @@ __global__ void __launch_bounds__(HALO ? kHaloRows : kBlock, MINB) k_fwd_euler_d
     const bool pf_lane = PREF && (threadIdx.x & 31) == 0;
     if (pf_lane) {
       sa.arr[0] = col; sa.esize[0] = 4;
-      sa.arr[1] = a.wdw[0]; sa.esize[1] = 8;
-      sa.arr[2] = a.wdw[1]; sa.esize[2] = 8;
-      sa.arr[3] = a.wldw; sa.esize[3] = 8;
-      sa.narr = (WQ || FLY) ? 4 : 3;
+      sa.arr[1] = a.wxydw; sa.esize[1] = 16;
+      sa.arr[2] = a.wldw; sa.esize[2] = 8;
+      sa.narr = NEEDL ? 3 : 2;
       s_lo = a.ell.slice_off[r >> 5];
       s_hi = a.ell.slice_off[(r >> 5) + 1];
       prefetch_chunk(sa, s_lo, s_hi, 0);
@@ -299,30 +356,34 @@ __global__ void __launch_bounds__(HALO ? kHaloRows : kBlock, MINB) k_fwd_euler_d
       if (pf_lane && (j % kPfSlots) == 0) prefetch_chunk(sa, s_lo, s_hi, j / kPfSlots + 2);
       const int64_t p = base + ((int64_t)j << 5);
       const int64_t c = __ldg(col + p);
-      fwd_accum<WT, WQ, FLY>(fwd_load<WT, WQ, FLY>(a, F, U, p, c), f, tx, ty, q);
+      fwd_accum<WT, NEEDL>(fwd_load<NEEDU, NEEDL>(a, F, U, p, c), sum);
     }
   } else if (len > 0) {
     int64_t c_next = len > 1 ? (int64_t)__ldg(col + base + 32) : 0;
-    FwdEntry cur = fwd_load<WT, WQ, FLY>(a, F, U, base, __ldg(col + base));
+    FwdEntry cur = fwd_load<NEEDU, NEEDL>(a, F, U, base, __ldg(col + base));
     for (int j = 0; j < len; ++j) {
       const int64_t p1 = base + ((int64_t)(j + 1) << 5);
       const int64_t c2 = j + 2 < len ? (int64_t)__ldg(col + p1 + 32) : 0;
       FwdEntry nxt;
-      if (j + 1 < len) nxt = fwd_load<WT, WQ, FLY>(a, F, U, p1, c_next);
-      fwd_accum<WT, WQ, FLY>(cur, f, tx, ty, q);
+      if (j + 1 < len) nxt = fwd_load<NEEDU, NEEDL>(a, F, U, p1, c_next);
+      fwd_accum<WT, NEEDL>(cur, sum);
       cur = nxt;
       c_next = c2;
     }
   }
   double du[4];
-  if (WT) du[0] = -dadd(dw::to_double(tx[1]), dw::to_double(ty[2]));
-  else du[0] = -dw::to_double(f[0]);
-#pragma unroll
-  for (int v = 1; v < 4; ++v) du[v] = -dw::to_double(f[v]);
+  if (WT) du[0] = -dw::sum_double(dw::second(sum.tx[0]), dw::first(sum.ty[1]));
+  else du[0] = -dw::sum_double(dw::first(sum.f0), dw::second(sum.f0));
+  du[1] = -dw::to_double(dw::first(sum.f12));
+  du[2] = -dw::to_double(dw::second(sum.f12));
+  du[3] = -dw::sum_double(dw::first(sum.f3), dw::second(sum.f3));
   double qv[4] = {0, 0, 0, 0};
   if (FLY) {
 #pragma unroll
-    for (int v = 0; v < 4; ++v) qv[v] = dw::to_double(q[v]);
+    for (int k = 0; k < 2; ++k) {
+      qv[2 * k] = dw::to_double(dw::first(sum.q[k]));
+      qv[2 * k + 1] = dw::to_double(dw::second(sum.q[k]));
+    }
   }
   if (FLY == 1) {
 #pragma unroll
@@ -330,9 +391,8 @@ __global__ void __launch_bounds__(HALO ? kHaloRows : kBlock, MINB) k_fwd_euler_d
   }
   if (WT) {
     float4* t4 = reinterpret_cast<float4*>(a.tdw) + i * 4;
-    float2 x[4], y[4];
-#pragma unroll
-    for (int v = 0; v < 4; ++v) { x[v] = dw::to_pair(tx[v]); y[v] = dw::to_pair(ty[v]); }
+    dw::DW2 t[4] = {dw::to_pair2(sum.tx[0]), dw::to_pair2(sum.tx[1]), dw::to_pair2(sum.ty[0]),
+                    dw::to_pair2(sum.ty[1])};
     if (a.fuse_eps) {
       // the viscosity of this node (FP64, as k_eps forms it from the partial du held
       // here) and s = eps * t written in place of t; this FP64 work overlaps the FP32
@@ -341,37 +401,25 @@ __global__ void __launch_bounds__(HALO ? kHaloRows : kBlock, MINB) k_fwd_euler_d
       pdl_wait();
       const double eps = visc::eps_value<4>(a.ea, i, du);
       if (a.ea.eps) a.ea.eps[i] = eps;
-      const float2 e2 = dw::split(eps);
+      const dw::DW2 e2 = dw::both(dw::split(eps));
 #pragma unroll
-      for (int v = 0; v < 4; ++v) { x[v] = dw::mul(e2, x[v]); y[v] = dw::mul(e2, y[v]); }
+      for (int k = 0; k < 4; ++k) t[k] = dw::mul(e2, t[k]);
     }
-    const float4 o[4] = {make_float4(x[0].x, x[0].y, x[1].x, x[1].y),
-                         make_float4(x[2].x, x[2].y, x[3].x, x[3].y),
-                         make_float4(y[0].x, y[0].y, y[1].x, y[1].y),
-                         make_float4(y[2].x, y[2].y, y[3].x, y[3].y)};
-    if (HINT) {
-      const uint64_t keep = l2_evict_last();
+    const uint64_t keep = HINT ? l2_evict_last() : 0;
 #pragma unroll
-      for (int k = 0; k < 4; ++k) st_hint(t4 + k, o[k], keep);
-    } else {
-#pragma unroll
-      for (int k = 0; k < 4; ++k) t4[k] = o[k];
+    for (int k = 0; k < 4; ++k) {
+      if (HINT) st_hint(t4 + k, dw::chunk(t[k]), keep);
+      else t4[k] = dw::chunk(t[k]);
     }
   }
   if (WQ) {
     float4* q4 = reinterpret_cast<float4*>(a.qdw) + i * 2;
-    float2 x[4];
+    const uint64_t keep = HINT ? l2_evict_last() : 0;
 #pragma unroll
-    for (int v = 0; v < 4; ++v) x[v] = dw::to_pair(q[v]);
-    const float4 o0 = make_float4(x[0].x, x[0].y, x[1].x, x[1].y);
-    const float4 o1 = make_float4(x[2].x, x[2].y, x[3].x, x[3].y);
-    if (HINT) {
-      const uint64_t keep = l2_evict_last();
-      st_hint(q4, o0, keep);
-      st_hint(q4 + 1, o1, keep);
-    } else {
-      q4[0] = o0;
-      q4[1] = o1;
+    for (int k = 0; k < 2; ++k) {
+      const float4 o = dw::chunk(dw::to_pair2(sum.q[k]));
+      if (HINT) st_hint(q4 + k, o, keep);
+      else q4[k] = o;
     }
   }
   if (FLY == 2) {
@@ -394,67 +442,64 @@ __global__ void __launch_bounds__(HALO ? kHaloRows : kBlock, MINB) k_fwd_euler_d
   }
 }
 
-// One entry of the transpose gather: weights and the neighbour's s = eps t and q records.
+// One entry of the transpose gather: weights and the neighbour's s = eps t (x part, y part;
+// two chunks each) and q chunks.
 struct RevEntry {
-  float2 wx, wy, wl;
-  F8 xa, ya, qq;
+  float4 wxy;
+  float2 wl;
+  float4 s[4], q[2];
 };
 
 template <bool RV, bool LAP>
-static __device__ __forceinline__ RevEntry rev_load(const RevArgs& a, const float* S,
-                                                    const float* Q, int64_t p, int64_t c) {
+static __device__ __forceinline__ RevEntry rev_load(const RevArgs& a, const float4* S,
+                                                    const float4* Q, int64_t p, int64_t c) {
   RevEntry e;
   if (RV) {
-    e.wx = __ldg(a.wdw[0] + p);
-    e.wy = __ldg(a.wdw[1] + p);
-    e.xa = ldg_f8(S + c * 16);
-    e.ya = ldg_f8(S + c * 16 + 8);
+    e.wxy = __ldg(a.wxydw + p);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) e.s[k] = __ldg(S + c * 4 + k);
   }
   if (LAP) {
     e.wl = __ldg(a.wldw + p);
-    e.qq = ldg_f8(Q + c * 8);
-  }
-  return e;
-}
-
-template <bool RV, bool LAP, bool HINT = false>
-static __device__ __forceinline__ RevEntry rev_load_halo(const RevArgs& a, const float4* sm,
-                                                         int hs, int64_t p, int lc,
-                                                         uint64_t pol = 0) {
-  RevEntry e;
-  constexpr int kq = RV ? 4 : 0;  // first chunk of the q record
-  if (RV) {
-    e.wx = HINT ? ldg_hint(a.wdw[0] + p, pol) : __ldg(a.wdw[0] + p);
-    e.wy = HINT ? ldg_hint(a.wdw[1] + p, pol) : __ldg(a.wdw[1] + p);
-    e.xa.lo = sm[lc];
-    e.xa.hi = sm[hs + lc];
-    e.ya.lo = sm[2 * hs + lc];
-    e.ya.hi = sm[3 * hs + lc];
-  }
-  if (LAP) {
-    e.wl = HINT ? ldg_hint(a.wldw + p, pol) : __ldg(a.wldw + p);
-    e.qq.lo = sm[kq * hs + lc];
-    e.qq.hi = sm[(kq + 1) * hs + lc];
+#pragma unroll
+    for (int k = 0; k < 2; ++k) e.q[k] = __ldg(Q + c * 2 + k);
   }
   return e;
 }
 
 template <bool RV, bool LAP>
-static __device__ __forceinline__ void rev_accum(const RevEntry& e, dw::Acc* sx, dw::Acc* sy,
-                                                 dw::Acc* sl) {
+static __device__ __forceinline__ RevEntry rev_load_halo(const Streamed& x, const float4* sm,
+                                                         int hs) {
+  RevEntry e;
+  constexpr int N = (RV ? 4 : 0) + (LAP ? 2 : 0), kq = RV ? 4 : 0;  // first chunk of the q record
   if (RV) {
-    const float2 X[4] = {lo2(e.xa.lo), hi2(e.xa.lo), lo2(e.xa.hi), hi2(e.xa.hi)};
-    const float2 Y[4] = {lo2(e.ya.lo), hi2(e.ya.lo), lo2(e.ya.hi), hi2(e.ya.hi)};
+    e.wxy = x.wxy;
 #pragma unroll
-    for (int v = 0; v < 4; ++v) {
-      dw::fma_acc(sx[v], e.wx, X[v]);
-      dw::fma_acc(sy[v], e.wy, Y[v]);
+    for (int k = 0; k < 4; ++k) e.s[k] = sm[halo_at<N>(k, x.lc, hs)];
+  }
+  if (LAP) {
+    e.wl = x.wl;
+#pragma unroll
+    for (int k = 0; k < 2; ++k) e.q[k] = sm[halo_at<N>(kq + k, x.lc, hs)];
+  }
+  return e;
+}
+
+// r: sums of Dx' s_x + Dy' s_y, l: of lap' q, two variables each
+template <bool RV, bool LAP>
+static __device__ __forceinline__ void rev_accum(const RevEntry& e, dw::Acc2* r, dw::Acc2* l) {
+  if (RV) {
+    const dw::DW2 wx = dw::both(dw::chunk_a(e.wxy)), wy = dw::both(dw::chunk_b(e.wxy));
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      dw::fma_acc2(r[k], wx, dw::pair2(e.s[k]));
+      dw::fma_acc2(r[k], wy, dw::pair2(e.s[2 + k]));
     }
   }
   if (LAP) {
-    const float2 Z[4] = {lo2(e.qq.lo), hi2(e.qq.lo), lo2(e.qq.hi), hi2(e.qq.hi)};
+    const dw::DW2 wl = dw::both(e.wl);
 #pragma unroll
-    for (int v = 0; v < 4; ++v) dw::fma_acc(sl[v], e.wl, Z[v]);
+    for (int k = 0; k < 2; ++k) dw::fma_acc2(l[k], wl, dw::pair2(e.q[k]));
   }
 }
 
@@ -465,15 +510,13 @@ template <bool RV, bool LAP, int PIPE, int MINB, bool PREF, bool HALO, bool HINT
 __global__ void __launch_bounds__(HALO ? kHaloRows : kBlock, MINB) k_rev_euler_dw(RevArgs a) {
   constexpr int NCH = (RV ? 4 : 0) + (LAP ? 2 : 0);
   const int64_t r = blockIdx.x * (int64_t)(HALO ? (int)blockDim.x : kBlock) + threadIdx.x;
-  const float* __restrict__ S = reinterpret_cast<const float*>(a.sdw);
-  const float* __restrict__ Q = reinterpret_cast<const float*>(a.qdw);
+  const float4* __restrict__ S = reinterpret_cast<const float4*>(a.sdw);
+  const float4* __restrict__ Q = reinterpret_cast<const float4*>(a.qdw);
   extern __shared__ float4 hsm[];
   bool staged = false;
   if (HALO && NCH > 0) {
-    const float4* S4 = reinterpret_cast<const float4*>(a.sdw);
-    const float4* Q4 = reinterpret_cast<const float4*>(a.qdw);
     staged = stage_halo<NCH>(a.ell, hsm, [&](int k, int64_t c) {
-      return (RV && k < 4) ? S4 + c * 4 + k : Q4 + c * 2 + (k - (RV ? 4 : 0));
+      return (RV && k < 4) ? S + c * 4 + k : Q + c * 2 + (k - (RV ? 4 : 0));
     });
   }
   if (r >= a.n) return;
@@ -481,9 +524,9 @@ __global__ void __launch_bounds__(HALO ? kHaloRows : kBlock, MINB) k_rev_euler_d
   const int64_t base = a.ell.slice_off[r >> 5] + (r & 31);
   const int len = a.ell.row_len[r];
   const int32_t* __restrict__ col = a.ell.col;
-  dw::Acc sx[4], sy[4], sl[4];
+  dw::Acc2 sr[2], sl[2];
 #pragma unroll
-  for (int v = 0; v < 4; ++v) { sx[v] = dw::zero(); sy[v] = dw::zero(); sl[v] = dw::zero(); }
+  for (int k = 0; k < 2; ++k) sr[k] = sl[k] = dw::zero2();
   const uint16_t* __restrict__ lcol = a.ell.lcol;
   const int hs = a.ell.halo_stride;
   if (HALO && staged) {
@@ -493,7 +536,7 @@ __global__ void __launch_bounds__(HALO ? kHaloRows : kBlock, MINB) k_rev_euler_d
     if (pf_lane) {
       int k = 0;
       sa.arr[k] = lcol; sa.esize[k++] = 2;
-      if (RV) { sa.arr[k] = a.wdw[0]; sa.esize[k++] = 8; sa.arr[k] = a.wdw[1]; sa.esize[k++] = 8; }
+      if (RV) { sa.arr[k] = a.wxydw; sa.esize[k++] = 16; }
       if (LAP) { sa.arr[k] = a.wldw; sa.esize[k++] = 8; }
       sa.narr = k;
       s_lo = a.ell.slice_off[r >> 5];
@@ -501,21 +544,43 @@ __global__ void __launch_bounds__(HALO ? kHaloRows : kBlock, MINB) k_rev_euler_d
       prefetch_chunk(sa, s_lo, s_hi, 0);
       prefetch_chunk(sa, s_lo, s_hi, 1);
     }
-    constexpr int UNR = PIPE < 1 ? 1 : PIPE;
+    constexpr int UNR = PIPE < 1 || PIPE == kPipelined ? 1 : PIPE;
     const uint64_t pol = HINT ? l2_evict_first() : 0;
-#pragma unroll UNR
-    for (int j = 0; j < len; ++j) {
-      if (pf_lane && (j % kPfSlots) == 0) prefetch_chunk(sa, s_lo, s_hi, j / kPfSlots + 2);
-      const int64_t p = base + ((int64_t)j << 5);
-      const int lc = HINT ? ldg_hint(lcol + p, pol) : __ldg(lcol + p);
-      rev_accum<RV, LAP>(rev_load_halo<RV, LAP, HINT>(a, hsm, hs, p, lc, pol), sx, sy, sl);
+    RowStream w{lcol + base, a.wxydw + base, a.wldw + base};
+    auto load = [&](Streamed& x, int j) { stream_load<RV, LAP, HINT>(x, w, j, pol); };
+    auto use = [&](const Streamed& x) {
+      rev_accum<RV, LAP>(rev_load_halo<RV, LAP>(x, hsm, hs), sr, sl);
+    };
+    if constexpr (PIPE == kPipelined) {
+      pipelined_row<3, Streamed>(len, load, use);
+    } else {
+      int j = 0;
+      for (; j + UNR <= len; j += UNR) {
+        if (pf_lane && (j % kPfSlots) < UNR) prefetch_chunk(sa, s_lo, s_hi, j / kPfSlots + 2);
+        Streamed x[UNR];
+#pragma unroll
+        for (int k = 0; k < UNR; ++k) load(x[k], k);
+#pragma unroll
+        for (int k = 0; k < UNR; ++k) use(x[k]);
+        w.lc += UNR * 32;
+        w.wxy += UNR * 32;
+        w.wl += UNR * 32;
+      }
+      for (; j < len; ++j) {
+        Streamed x;
+        load(x, 0);
+        use(x);
+        w.lc += 32;
+        w.wxy += 32;
+        w.wl += 32;
+      }
     }
   } else if (PIPE == 0) {
 #pragma unroll 1
     for (int j = 0; j < len; ++j) {
       const int64_t p = base + ((int64_t)j << 5);
       const int64_t c = __ldg(col + p);
-      rev_accum<RV, LAP>(rev_load<RV, LAP>(a, S, Q, p, c), sx, sy, sl);
+      rev_accum<RV, LAP>(rev_load<RV, LAP>(a, S, Q, p, c), sr, sl);
     }
   } else if (PIPE == 2 || (HALO && PIPE > 2)) {
     SliceArrays sa{};
@@ -524,7 +589,7 @@ __global__ void __launch_bounds__(HALO ? kHaloRows : kBlock, MINB) k_rev_euler_d
     if (pf_lane) {
       int k = 0;
       sa.arr[k] = col; sa.esize[k++] = 4;
-      if (RV) { sa.arr[k] = a.wdw[0]; sa.esize[k++] = 8; sa.arr[k] = a.wdw[1]; sa.esize[k++] = 8; }
+      if (RV) { sa.arr[k] = a.wxydw; sa.esize[k++] = 16; }
       if (LAP) { sa.arr[k] = a.wldw; sa.esize[k++] = 8; }
       sa.narr = k;
       s_lo = a.ell.slice_off[r >> 5];
@@ -537,7 +602,7 @@ __global__ void __launch_bounds__(HALO ? kHaloRows : kBlock, MINB) k_rev_euler_d
       if (pf_lane && (j % kPfSlots) == 0) prefetch_chunk(sa, s_lo, s_hi, j / kPfSlots + 2);
       const int64_t p = base + ((int64_t)j << 5);
       const int64_t c = __ldg(col + p);
-      rev_accum<RV, LAP>(rev_load<RV, LAP>(a, S, Q, p, c), sx, sy, sl);
+      rev_accum<RV, LAP>(rev_load<RV, LAP>(a, S, Q, p, c), sr, sl);
     }
   } else if (len > 0) {
     int64_t c_next = len > 1 ? (int64_t)__ldg(col + base + 32) : 0;
@@ -547,7 +612,7 @@ __global__ void __launch_bounds__(HALO ? kHaloRows : kBlock, MINB) k_rev_euler_d
       const int64_t c2 = j + 2 < len ? (int64_t)__ldg(col + p1 + 32) : 0;
       RevEntry nxt;
       if (j + 1 < len) nxt = rev_load<RV, LAP>(a, S, Q, p1, c_next);
-      rev_accum<RV, LAP>(cur, sx, sy, sl);
+      rev_accum<RV, LAP>(cur, sr, sl);
       cur = nxt;
       c_next = c2;
     }
@@ -559,8 +624,9 @@ __global__ void __launch_bounds__(HALO ? kHaloRows : kBlock, MINB) k_rev_euler_d
 #pragma unroll
   for (int v = 0; v < 4; ++v) {
     double d = dp[v];
-    if (RV) d = dsub(dsub(d, dw::to_double(sx[v])), dw::to_double(sy[v]));
-    if (LAP) d = fma(-a.hv_gamma, dw::to_double(sl[v]), d);
+    if (RV) d = dsub(d, dw::to_double(v & 1 ? dw::second(sr[v >> 1]) : dw::first(sr[v >> 1])));
+    if (LAP)
+      d = fma(-a.hv_gamma, dw::to_double(v & 1 ? dw::second(sl[v >> 1]) : dw::first(sl[v >> 1])), d);
     if (a.hvf) d = dadd(d, a.hvf[i * 4 + v]);
     du[v] = d;
   }
@@ -581,7 +647,9 @@ float2 gm1_pair(double gamma) {
   return make_float2(h, (float)(gm1 - (double)h));
 }
 
-bool dw_fwd_fuses(int variant) { return variant == 7 || variant == 11 || variant == 12; }
+bool dw_fwd_fuses(int variant) {
+  return variant == 7 || variant == 9 || variant == 11 || variant == 12;
+}
 
 void launch_prep_euler_dw(int64_t n, double gamma, const double* u, float2* F, float2* U,
                           cudaStream_t s) {
@@ -600,11 +668,12 @@ namespace {
 // the slice's streamed arrays prefetched into L2 ahead of use, 5 = variant 2 with it,
 // 6 / 7 = neighbour records staged per row group in shared memory (one / two entries per
 // iteration, registers capped at three blocks of kHaloRows per SM), 8 = variant 7 capped
-// at four blocks, 9 / 11 = staged with four / three entries per iteration, 10 = variant 7
-// with the streamed position and weight arrays prefetched into L2 (as variant 4), 12 =
-// variant 7 with L2 eviction-priority hints (streamed arrays evict-first; the forward
-// gather's t, q and partial du evict-last for the transpose gather).  Without halos
-// (not built) the staged variants run as variant 2.
+// at four blocks, 9 = staged with the streamed loads in software pipeline (pipelined_row,
+// groups of three entries, registers capped at two blocks), 11 = staged with three entries
+// per iteration, 10 = variant 7 with the streamed position and weight arrays prefetched into
+// L2 (as variant 4), 12 = variant 7 with L2 eviction-priority hints (streamed arrays
+// evict-first; the forward gather's t, q and partial du evict-last for the transpose gather).
+// Without halos (not built) the staged variants run as variant 2.
 // A staged launch: one block per row group, NCH chunks of the layout's longest list
 // in dynamic shared memory (above 48 KB that needs a per-kernel opt-in, made once per
 // kernel and device).
@@ -629,13 +698,14 @@ void launch_staged(void (*k)(Args), const Args& a, int nch, int64_t n, cudaStrea
 template <bool WT, bool WQ, int FLY>
 void fwd_variant(const FwdArgs& a, int variant, int64_t n, cudaStream_t s) {
   const unsigned g = grid_for(n, kBlock);
-  constexpr int nch = (WT || WQ || FLY) ? 6 : 4;
+  constexpr int nch = kFwdChunks<WT || WQ || FLY != 0>;
   const bool pdl = a.pdl != 0;
   if (variant >= 6 && !a.ell.halo_off) variant = 2;
   if (a.fuse_flux && a.ell.halo_off && dw_fwd_fuses(variant)) {
     MFT_REQUIRE(a.ustate && a.err, MFT_ERR_STATE, "fused staging needs the state and error word");
     switch (variant) {
       case 7: launch_staged(k_fwd_euler_dw<WT, WQ, FLY, 2, 3, false, true, false, true>, a, nch, n, s, pdl); break;
+      case 9: launch_staged(k_fwd_euler_dw<WT, WQ, FLY, kPipelined, 2, false, true, false, true>, a, nch, n, s, pdl); break;
       case 11: launch_staged(k_fwd_euler_dw<WT, WQ, FLY, 3, 3, false, true, false, true>, a, nch, n, s, pdl); break;
       default: launch_staged(k_fwd_euler_dw<WT, WQ, FLY, 2, 3, false, true, true, true>, a, nch, n, s, pdl); break;
     }
@@ -650,7 +720,7 @@ void fwd_variant(const FwdArgs& a, int variant, int64_t n, cudaStream_t s) {
     case 6: launch_staged(k_fwd_euler_dw<WT, WQ, FLY, 0, 3, false, true>, a, nch, n, s, pdl); break;
     case 7: launch_staged(k_fwd_euler_dw<WT, WQ, FLY, 2, 3, false, true>, a, nch, n, s, pdl); break;
     case 8: launch_staged(k_fwd_euler_dw<WT, WQ, FLY, 2, 4, false, true>, a, nch, n, s, pdl); break;
-    case 9: launch_staged(k_fwd_euler_dw<WT, WQ, FLY, 4, 3, false, true>, a, nch, n, s, pdl); break;
+    case 9: launch_staged(k_fwd_euler_dw<WT, WQ, FLY, kPipelined, 2, false, true>, a, nch, n, s, pdl); break;
     case 10: launch_staged(k_fwd_euler_dw<WT, WQ, FLY, 2, 3, true, true>, a, nch, n, s, pdl); break;
     case 11: launch_staged(k_fwd_euler_dw<WT, WQ, FLY, 3, 3, false, true>, a, nch, n, s, pdl); break;
     case 12: launch_staged(k_fwd_euler_dw<WT, WQ, FLY, 2, 3, false, true, true>, a, nch, n, s, pdl); break;
@@ -672,7 +742,7 @@ void rev_variant(const RevArgs& a, int variant, int64_t n, cudaStream_t s) {
     case 6: launch_staged(k_rev_euler_dw<RV, LAP, 0, 3, false, true>, a, nch, n, s); break;
     case 7: launch_staged(k_rev_euler_dw<RV, LAP, 2, 3, false, true>, a, nch, n, s); break;
     case 8: launch_staged(k_rev_euler_dw<RV, LAP, 2, 4, false, true>, a, nch, n, s); break;
-    case 9: launch_staged(k_rev_euler_dw<RV, LAP, 4, 3, false, true>, a, nch, n, s); break;
+    case 9: launch_staged(k_rev_euler_dw<RV, LAP, kPipelined, 2, false, true>, a, nch, n, s); break;
     case 10: launch_staged(k_rev_euler_dw<RV, LAP, 2, 3, true, true>, a, nch, n, s); break;
     case 11: launch_staged(k_rev_euler_dw<RV, LAP, 3, 3, false, true>, a, nch, n, s); break;
     case 12: launch_staged(k_rev_euler_dw<RV, LAP, 2, 3, false, true, true>, a, nch, n, s); break;

@@ -244,8 +244,8 @@ __global__ void __launch_bounds__(HALO ? kHaloRows : kBlock) k_rev_f32(RevArgs a
       if (V == 4) {
         float4 xs, ys;
         if (HALO && staged) {
-          xs = hsm[c];
-          ys = hsm[hs + c];
+          xs = hsm[halo_at<NCH>(0, c, hs)];
+          ys = hsm[halo_at<NCH>(1, c, hs)];
         } else {
           const F8 st = ldg_f8(a.s32 + (int64_t)c * 8);
           xs = st.lo;
@@ -265,7 +265,7 @@ __global__ void __launch_bounds__(HALO ? kHaloRows : kBlock) k_rev_f32(RevArgs a
       const float wl = __ldg(a.wl32 + p);
       if (V == 4) {
         const float4 qq = (HALO && staged)
-                              ? hsm[(RV ? 2 : 0) * hs + c]
+                              ? hsm[halo_at<NCH>(RV ? 2 : 0, c, hs)]
                               : __ldg(reinterpret_cast<const float4*>(a.q32) + c);
         sl[0] = fmaf(wl, qq.x, sl[0]); sl[1] = fmaf(wl, qq.y, sl[1]);
         sl[2] = fmaf(wl, qq.z, sl[2]); sl[3] = fmaf(wl, qq.w, sl[3]);

@@ -165,7 +165,7 @@ static __device__ __forceinline__ void finish_node(const Epilogue& ep, int64_t i
     bool bad = false;
 #pragma unroll
     for (int v = 0; v < V; ++v)
-      bad |= ((__double_as_longlong(o[v]) >> 52) & 0x7FF) == 0x7FF;
+      bad |= (__double2hiint(o[v]) & 0x7FF00000) == 0x7FF00000;
     if (bad) atomicMax(ep.err, (int)MFT_ERR_NONFINITE);
   }
 #pragma unroll

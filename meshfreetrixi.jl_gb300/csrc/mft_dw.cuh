@@ -8,7 +8,7 @@
 //     e = a_h b_h - p exactly = fma(a_h, b_h, -p)  (Dekker 1971, with an FMA);
 //   * the cross terms a_h b_l + a_l b_h folded into e (a_l b_l < 2^-48 |ab| is dropped);
 //   * the exact sum of the running high part and p by Knuth's TwoSum (branch-free),
-//     whose rounding error joins e in a float carry.
+//     whose rounding error joins e in a float carry (fma_acc).
 // This is the compensated dot product "Dot2" of Ogita, Rump and Oishi (SIAM J. Sci.
 // Comput. 26(6), 2005) on double-word inputs (Joldes, Muller and Popescu, ACM TOMS
 // 44(2), 2017).  With u = 2^-24, a length-n sum of products carries the inputs' split
@@ -31,11 +31,7 @@ using fpconv::d2f;
 using fpconv::f2d;
 
 // x -> (h, l): h = RN32(x), l = RN32(x - h) (x - h is exact in FP64).
-static __device__ __forceinline__ float2 split(double x) {
-  const float h = d2f(x);
-  const float l = d2f(__dsub_rn(x, f2d(h)));
-  return make_float2(h, l);
-}
+static __device__ __forceinline__ float2 split(double x) { return fpconv::split(x); }
 
 static __device__ __forceinline__ double value(float2 a) {
   return __dadd_rn(f2d(a.x), f2d(a.y));
@@ -49,17 +45,20 @@ struct Acc {
 
 static __device__ __forceinline__ Acc zero() { return Acc{0.f, 0.f}; }
 
-// acc += a * b (a, b double-word)
+// acc += a * b (a, b double-word), 10 operations.  With p = RN(a_h b_h), t = RN(s + p) and
+// b' = RN(t - s) (Knuth's TwoSum; nb = -b'), the sum's rounding error is (s - (t - b')) +
+// (p - b') exactly and the product's a_h b_h - p, so fma(a_h, b_h, nb) = RN(a_h b_h - b') is
+// the product's error and the second part of the sum's in one operation.
 static __device__ __forceinline__ void fma_acc(Acc& acc, float2 a, float2 b) {
   const float p = __fmul_rn(a.x, b.x);
-  float e = fmaf(a.x, b.x, -p);
+  const float t = __fadd_rn(acc.s, p);
+  const float nb = __fsub_rn(acc.s, t);
+  float e = fmaf(a.x, b.x, nb);
   e = fmaf(a.x, b.y, e);
   e = fmaf(a.y, b.x, e);
-  const float t = __fadd_rn(acc.s, p);
-  const float bp = __fsub_rn(t, acc.s);
-  const float err = __fadd_rn(__fsub_rn(acc.s, __fsub_rn(t, bp)), __fsub_rn(p, bp));
+  e = __fadd_rn(e, __fsub_rn(acc.s, __fadd_rn(t, nb)));
   acc.s = t;
-  acc.c = __fadd_rn(acc.c, __fadd_rn(err, e));
+  acc.c = __fadd_rn(acc.c, e);
 }
 
 // The accumulated value rounded once to FP64.
@@ -136,6 +135,105 @@ static __device__ __forceinline__ void euler_flux_vjp(float2 gm1, const float2* 
   ub[1] = add(add(add(gx[0], mul(gx[1], v1)), add(mul(gx[2], v2), neg(mul(hp, v1)))), mul(v1b, ri));
   ub[2] = add(add(add(gy[0], mul(gy[1], v1)), add(mul(gy[2], v2), neg(mul(hp, v2)))), mul(v2b, ri));
   ub[3] = add(add(mul(gx[3], v1), mul(gy[3], v2)), mul(gm1, pb));
+}
+
+// ---------------------------------------------------------------- two at a time
+// The same operations on two double-word values at once with the packed FP32 instructions
+// (add / sub / mul / fma .f32x2: two roundings per instruction, each as the scalar one).
+// They run at the scalar instructions' rate per operation (measured 16.5 T packed against
+// 28-39 T scalar instructions per second and GPU) but take half the issue slots, which the
+// gathers need for their loads.
+typedef unsigned long long f32x2;
+
+static __device__ __forceinline__ f32x2 pk(float x, float y) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+  return r;
+}
+static __device__ __forceinline__ float2 unpk(f32x2 v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+static __device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+static __device__ __forceinline__ f32x2 sub2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+static __device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+
+// RN(a b), as the multiply-add a b + (-0) with the -0 read from constant memory: the compiler
+// contracts a packed multiplication and the packed addition that reads it into one multiply-add
+// (also with .rn on both, with a literal -0 and without -fmad; the scalar instructions keep
+// their .rn), which would break the error-free steps.
+static __constant__ unsigned long long kNegZero2 = 0x8000000080000000ull;
+static __device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) { return fma2(a, b, kNegZero2); }
+
+// Two double-word values a, b: (a_h, b_h) and (a_l, b_l).  In memory the 16-byte chunk
+// (a_h, b_h, a_l, b_l), so that a chunk's load leaves them in register pairs.
+struct DW2 {
+  f32x2 h, l;
+};
+static __device__ __forceinline__ DW2 pair2(float4 c) { return DW2{pk(c.x, c.y), pk(c.z, c.w)}; }
+static __device__ __forceinline__ DW2 pair2(float2 a, float2 b) {
+  return DW2{pk(a.x, b.x), pk(a.y, b.y)};
+}
+static __device__ __forceinline__ DW2 both(float2 a) { return pair2(a, a); }
+static __device__ __forceinline__ float4 chunk(float2 a, float2 b) {
+  return make_float4(a.x, b.x, a.y, b.y);
+}
+static __device__ __forceinline__ float4 chunk(DW2 v) {
+  const float2 h = unpk(v.h), l = unpk(v.l);
+  return make_float4(h.x, h.y, l.x, l.y);
+}
+static __device__ __forceinline__ float2 chunk_a(float4 c) { return make_float2(c.x, c.z); }
+static __device__ __forceinline__ float2 chunk_b(float4 c) { return make_float2(c.y, c.w); }
+
+struct Acc2 {
+  f32x2 s, c;
+};
+static __device__ __forceinline__ Acc2 zero2() { return Acc2{0ull, 0ull}; }
+static __device__ __forceinline__ void fma_acc2(Acc2& acc, DW2 a, DW2 b) {
+  const f32x2 p = mul2(a.h, b.h);
+  const f32x2 t = add2(acc.s, p);
+  const f32x2 nb = sub2(acc.s, t);
+  f32x2 e = fma2(a.h, b.h, nb);
+  e = fma2(a.h, b.l, e);
+  e = fma2(a.l, b.h, e);
+  e = add2(e, sub2(acc.s, add2(t, nb)));
+  acc.s = t;
+  acc.c = add2(acc.c, e);
+}
+static __device__ __forceinline__ Acc first(Acc2 a) { return Acc{unpk(a.s).x, unpk(a.c).x}; }
+static __device__ __forceinline__ Acc second(Acc2 a) { return Acc{unpk(a.s).y, unpk(a.c).y}; }
+
+static __device__ __forceinline__ DW2 to_pair2(Acc2 a) {
+  const f32x2 t = add2(a.s, a.c);
+  const f32x2 bp = sub2(t, a.s);
+  return DW2{t, add2(sub2(a.s, sub2(t, bp)), sub2(a.c, bp))};
+}
+// The sum of two accumulated values rounded to FP64: the pairs added in double-word
+// arithmetic (add, about 2 u^2 of their sum), one FP64 addition.
+static __device__ __forceinline__ double sum_double(Acc a, Acc b) {
+  return value(add(to_pair(a), to_pair(b)));
+}
+
+static __device__ __forceinline__ DW2 mul(DW2 a, DW2 b) {
+  const f32x2 p = mul2(a.h, b.h);
+  f32x2 e = fma2(a.h, b.h, sub2(kNegZero2, p));  // -0 - p = -p
+  e = fma2(a.h, b.l, e);
+  e = fma2(a.l, b.h, e);
+  const f32x2 t = add2(p, e);
+  return DW2{t, sub2(e, sub2(t, p))};
 }
 
 }  // namespace dw

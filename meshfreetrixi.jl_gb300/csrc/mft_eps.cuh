@@ -6,6 +6,7 @@
 #include <cuda_runtime.h>
 #include <math.h>
 
+#include "mft_fpbits.h"
 #include "mft_internal.cuh"
 
 namespace mft {
@@ -28,19 +29,26 @@ static __device__ __forceinline__ double jl_min(double a, double b) {
   return jl_isless(b, a) ? b : a;
 }
 
-// Julia's max for arguments that are +0 or larger, or NaN (NaN propagates as a + b):
-// without NaN the larger value is the larger IEEE bit pattern, so no FP64 comparison
-// is issued.
+// The tests below work on 32-bit words of the IEEE patterns: an FP64 comparison takes a slot
+// of the slow FP64 pipe, and the compiler turns tests for NaN or infinity on a 64-bit pattern
+// back into one.
+static __device__ __forceinline__ bool nan_words(int hi, int lo) {
+  const unsigned h = (unsigned)hi & 0x7FFFFFFFu;
+  return h > 0x7FF00000u || (h == 0x7FF00000u && lo != 0);
+}
+// Julia's max for arguments that are +0 or larger, or NaN (NaN propagates): without NaN the
+// larger value is the larger pattern.
 static __device__ __forceinline__ double jl_max_nonneg(double a, double b) {
-  const long long ia = __double_as_longlong(a), ib = __double_as_longlong(b);
-  const long long inf = 0x7FF0000000000000LL;
-  if ((ia & 0x7FFFFFFFFFFFFFFFLL) > inf || (ib & 0x7FFFFFFFFFFFFFFFLL) > inf) return a + b;
-  return ib > ia ? b : a;
+  const int ha = __double2hiint(a), la = __double2loint(a);
+  const int hb = __double2hiint(b), lb = __double2loint(b);
+  const bool b_larger = hb > ha || (hb == ha && (unsigned)lb > (unsigned)la);
+  const bool take_b = nan_words(ha, la) ? false : nan_words(hb, lb) ? true : b_larger;
+  return __hiloint2double(take_b ? hb : ha, take_b ? lb : la);
 }
 
 // isnan(x) || isinf(x) on the exponent bits
 static __device__ __forceinline__ bool not_finite(double x) {
-  return ((__double_as_longlong(x) >> 52) & 0x7FF) == 0x7FF;
+  return (__double2hiint(x) & 0x7FF00000) == 0x7FF00000;
 }
 
 // 1 / x within an ulp: an FP32 reciprocal estimate refined by two Newton steps
@@ -124,12 +132,28 @@ static __device__ __forceinline__ double eps_value(const EpsArgs& a, int64_t i,
   // bound a node at rest qualifies too).  A NaN energy, or a density so small that
   // 1 / rho overflows (0 * inf in a velocity), would make eps_uw NaN: no shortcut then.
   // The final comparison is on bit patterns of values >= 0 (or NaN, which fails it).
+  // The same test in FP32 first (the FP64 pipe is the scarce one): its terms carry less than
+  // 1e-5 of relative error (mm <= E rho is asked with that margin too, so the difference keeps
+  // half of E rho), so lhs < (1 - 1e-4) rhs in FP32 proves the FP64 inequality; the ranges keep
+  // the FP32 terms normal (lhs may underflow: it is then below rhs).
   bool done = false;
+  if (V == 4 && rv_finite) {
+    const float rf = fpconv::d2f(rho), ef = fpconv::d2f(en);
+    const float f1 = fpconv::d2f(m1), f2 = fpconv::d2f(m2), uf = fpconv::d2f(uwc);
+    const float er = fpconv::d2f(eps_rv) * rf;
+    const float mm = f1 * f1 + f2 * f2, erho = ef * rf;
+    float w = mm;
+    if (mm <= 0.99999f * erho) w = mm + a.gg1_32 * (erho - 0.5f * mm);
+    const float rhs = uf * uf * w;
+    if (rf >= 1e-6f && uf > 0.0f && ef == ef && w >= 1e-18f && rhs >= 1e-30f && rhs <= 1e30f &&
+        er * er < 0.9999f * rhs)
+      return eps_rv;
+  }
   const double kb = a.seg_h ? dmul(dmul(uwc, uwc), (1.0 - 1e-12) / (1.0 + 1e-12)) : a.uw_bound;
   const long long bits_rho = __double_as_longlong(rho);
-  const long long bits_en = __double_as_longlong(en) & 0x7FFFFFFFFFFFFFFFLL;
   if (V == 4 && rv_finite && bits_rho >= 0x01A56E1FC2F8F359LL /* 1e-300 */ &&
-      __double_as_longlong(uwc) > 0 && bits_en <= 0x7FF0000000000000LL) {
+      __double_as_longlong(uwc) > 0 &&
+      !nan_words(__double2hiint(en), __double2loint(en))) {
     const double er = dmul(eps_rv, rho);
     const double lhs = dmul(er, er);
     const double mm = dadd(dmul(m1, m1), dmul(m2, m2));

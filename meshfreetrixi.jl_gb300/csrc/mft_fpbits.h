@@ -69,6 +69,25 @@ MFT_FPBITS_FN bool d2f_bits(uint32_t hi, uint32_t lo, uint32_t* out) {
   return false;  // below the normal floats, above them, infinity, NaN
 }
 
+// (hi, lo): the words of a double x.  On success *h is the bits of RN32(x) and
+// x - RN32(x) = *rem * 2^k exactly, |*rem| <= 2^28, with *scale the bits of the float 2^k; then
+// RN32(x - RN32(x)) = (float)*rem * 2^k (the conversion rounds, the product is exact).
+// Declines where that product could be subnormal, RN32(x) is not a normal float, or x is zero.
+MFT_FPBITS_FN bool split_words(uint32_t hi, uint32_t lo, uint32_t* h, int32_t* rem,
+                               uint32_t* scale) {
+  const uint32_t e = (hi >> 20) & 0x7FFu;
+  if (e - 949u >= 201u) return false;  // 2^-74 <= |x| < 2^127
+  uint32_t r = ((e - 896u) << 23) | ((hi & 0xFFFFFu) << 3) | (lo >> 29);
+  const uint32_t cut = lo & 0x1FFFFFFFu, half = 0x10000000u;
+  const uint32_t up = (cut > half || (cut == half && (r & 1u))) ? 1u : 0u;
+  r += up;
+  const int32_t d = (int32_t)cut - (up ? 0x20000000 : 0);
+  *h = r | (hi & 0x80000000u);
+  *rem = (hi & 0x80000000u) ? -d : d;
+  *scale = (e - 948u) << 23;  // 2^(e - 1075)
+  return true;
+}
+
 }  // namespace fpbits
 
 #if defined(__CUDACC__)
@@ -85,6 +104,18 @@ static __device__ __forceinline__ float d2f(double x) {
   if (fpbits::d2f_bits((uint32_t)__double2hiint(x), (uint32_t)__double2loint(x), &r))
     return __uint_as_float(r);
   return __double2float_rn(x);
+}
+// x -> (h, l), h = RN32(x), l = RN32(x - h), without the FP64 pipe in the range split_words
+// takes.
+static __device__ __forceinline__ float2 split(double x) {
+  uint32_t h, scale;
+  int32_t rem;
+  if (fpbits::split_words((uint32_t)__double2hiint(x), (uint32_t)__double2loint(x), &h, &rem,
+                          &scale))
+    return make_float2(__uint_as_float(h),
+                       __fmul_rn(__int2float_rn(rem), __uint_as_float(scale)));
+  const float hf = d2f(x);
+  return make_float2(hf, d2f(__dsub_rn(x, f2d(hf))));
 }
 }  // namespace fpconv
 #endif

@@ -41,6 +41,13 @@ static __device__ __forceinline__ float2 ldg_hint(const float2* ptr, uint64_t po
       : "l"(ptr), "l"(pol));
   return v;
 }
+static __device__ __forceinline__ float4 ldg_hint(const float4* ptr, uint64_t pol) {
+  float4 v;
+  asm("ld.global.nc.L2::cache_hint.v4.f32 {%0, %1, %2, %3}, [%4], %5;\n"
+      : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+      : "l"(ptr), "l"(pol));
+  return v;
+}
 static __device__ __forceinline__ int ldg_hint(const uint16_t* ptr, uint64_t pol) {
   unsigned short v;
   asm("ld.global.nc.L2::cache_hint.u16 %0, [%1], %2;\n" : "=h"(v) : "l"(ptr), "l"(pol));
@@ -57,10 +64,20 @@ static __device__ __forceinline__ void st_hint(double2* ptr, double2 v, uint64_t
                : "memory");
 }
 
+// Shared-memory place (in 16-byte chunks) of chunk k of list entry q, NCH chunks per record
+// and hs the longest list: record-major in runs of an odd number of chunks (an odd count as it
+// is; 3 + 3 for six, 3 + 1 for four, 1 + 1 for two), so that one multiplication addresses a run and its other
+// chunks are immediate offsets, while lanes reading one chunk of different records still spread
+// over the bank groups by q mod 8 (an odd stride permutes them).
+template <int NCH>
+static __device__ __forceinline__ int halo_at(int k, int q, int hs) {
+  constexpr int A = NCH % 2 ? NCH : NCH == 6 || NCH == 4 ? 3 : 1, B = NCH > A ? NCH - A : 1;
+  return k < A ? q * A + k : hs * A + q * B + (k - A);
+}
+
 // Stages the neighbour records of this block's row group (the group's halo list) into
 // shared memory: NCH 16-byte chunks per record, chunk k of list entry q at
-// sm[k * ell.halo_stride + q] (chunk-major, so that lanes reading one chunk of different
-// records spread over the banks).  chunk(k, c) is the address of chunk k of node c's
+// sm[halo_at<NCH>(k, q, ell.halo_stride)].  chunk(k, c) is the address of chunk k of node c's
 // record.  Consecutive threads copy consecutive chunks of one record, so each record
 // arrives in whole sectors.  Returns false (nothing staged) when the group has no list.
 // Every thread of the block must call it (it ends with a block barrier); the block is one
@@ -72,12 +89,41 @@ __device__ __forceinline__ bool stage_halo(const EllView& ell, float4* sm, Chunk
   if (nh <= 0) return false;  // block-uniform
   for (int q = threadIdx.x; q < nh * NCH; q += blockDim.x) {
     const int rec = q / NCH, k = q - rec * NCH;
-    cp_async16(sm + k * ell.halo_stride + rec,
+    cp_async16(sm + halo_at<NCH>(k, rec, ell.halo_stride),
                chunk(k, (int64_t)__ldg(ell.halo_col + h0 + rec)));
   }
   cp_async_wait_all();
   __syncthreads();
   return true;
+}
+
+// A staged row's loop with the streamed loads in software pipeline: Entry (positions, weights;
+// load(e, j) requests entry j's) in two register groups of G; a group's loads are issued before
+// the other group is used, so that a group's arithmetic covers their latency.  The entries are
+// used in order, use(e).
+template <int G, typename Entry, typename Load, typename Use>
+__device__ __forceinline__ void pipelined_row(int len, Load load, Use use) {
+  Entry e[2][G];
+  auto get = [&](Entry* x, int g) {
+#pragma unroll
+    for (int k = 0; k < G; ++k) load(x[k], g * G + k);
+  };
+  const int ng = len / G;
+  if (ng > 0) get(e[0], 0);
+  for (int g = 0; g < ng; g += 2) {
+    if (g + 1 < ng) get(e[1], g + 1);
+#pragma unroll
+    for (int k = 0; k < G; ++k) use(e[0][k]);
+    if (g + 2 < ng) get(e[0], g + 2);
+    if (g + 1 < ng) {
+#pragma unroll
+      for (int k = 0; k < G; ++k) use(e[1][k]);
+    }
+  }
+  for (int j = ng * G; j < len; ++j) {
+    load(e[0][0], j);
+    use(e[0][0]);
+  }
 }
 
 }  // namespace

@@ -194,11 +194,12 @@ struct Epilogue {
 void launch_aos_from_soa(const double* soa, double* aos, int64_t n, int V, cudaStream_t s);
 void launch_soa_from_aos(const double* aos, double* soa, int64_t n, int V, cudaStream_t s);
 void launch_aos_to_f32(const double* aos, float* a32, int64_t count, cudaStream_t s);
-// out[pos[e]] = v[e] (and out32[pos[e]] = (float) v[e] when out32 is not null, and
-// outdw[pos[e]] = the double-word pair of v[e] when outdw is not null): the operator
-// values of structure entry e placed at their sliced-ELL element.
+// out[pos[e]] = v[e] (and out32[pos[e]] = (float) v[e] when out32 is not null, and the
+// double-word pair (h, l) of v[e] when outdw is not null): the operator values of structure
+// entry e placed at their sliced-ELL element.  outdw: part < 0 writes the pair h, l; part 0
+// or 1 the first or second value of a chunk of two (dw::chunk), four floats per element.
 void launch_scatter_values(int64_t nnz, const int64_t* pos, const double* v, double* out,
-                           float* out32, float2* outdw, cudaStream_t s);
+                           float* out32, float2* outdw, int part, cudaStream_t s);
 
 // One pointer per variable (pinned host memory mapped for the device, or device memory).
 struct VarPtrs {
@@ -232,6 +233,7 @@ struct EpsArgs {
   double rv_coef;          // (0.5 * c_rv) * (h * h)
   double uw_bound;         // uw_coef^2 (1 - 1e-12) / (1 + 1e-12): the eps_uw bound's factor
   double gg1;              // gamma (gamma - 1): the sound speed's part of that bound
+  float gg1_32;
   // FP32 form: the FP32 shadow of u and the FP32 factors, formed by launch_eps in the
   // FP32 kernel's operation order
   const float* u32;
@@ -281,7 +283,8 @@ struct FwdArgs {
   Epilogue ep;
   // FP64 form in double-word arithmetic (Euler): weights, fluxes and states as (h, l)
   // float pairs; t and q are written as pairs, du_p / hvf in FP64
-  const float2* wdw[3];
+  const float4* wxydw;  // D_x and D_y as chunks (w_x, w_y) (mft_dw.cuh)
+  const float2* wzdw;   // 3D: D_z as pairs
   const float2* wldw;
   const float2* Fdw;    // n x 2V pairs
   const float2* udw;    // n x V pairs
@@ -309,8 +312,8 @@ void launch_fwd_f64(const FwdArgs& a, cudaStream_t s);
 // advection with the flux a_d u formed at the neighbour).
 void launch_flux_euler3d(int64_t n, double gamma, const double* u, double* F, cudaStream_t s);
 void launch_fwd3(const FwdArgs& a, cudaStream_t s);
-// The same for 3D Euler in double-word arithmetic: flux pairs (n x 16 float2, the 15 of
-// F_x, F_y, F_z and one pad) and the gather over the weight pairs a.wdw[0..2].
+// The same for 3D Euler in double-word arithmetic: flux records (n x 14 float2, seven
+// chunks) and the gather over the weights a.wxydw, a.wzdw.
 void launch_prep_euler3d_dw(int64_t n, double gamma, const double* u, float2* F,
                             cudaStream_t s);
 void launch_fwd3_dw(const FwdArgs& a, cudaStream_t s);
@@ -322,7 +325,7 @@ void launch_prep_euler_dw(int64_t n, double gamma, const double* u, float2* F, f
 constexpr int kDwVariants = 13;
 void launch_fwd_dw(const FwdArgs& a, int variant, cudaStream_t s);
 // Whether forward variant `variant` forms the flux pairs while staging when a.fuse_flux
-// is set (the staged variants 7, 11 and 12).
+// is set (the staged variants 7, 9, 11 and 12).
 bool dw_fwd_fuses(int variant);
 // The pairs of gamma - 1 (h = RN32(gamma - 1), l = RN32 of the remainder).
 float2 gm1_pair(double gamma);
@@ -367,7 +370,7 @@ struct RevArgs {
   double* du_p_out;
   float* du_p_out32;
   Epilogue ep;
-  const float2* wdw[3];  // double-word FP64 form: weights on the reverse layout
+  const float4* wxydw;   // double-word FP64 form: weights on the reverse layout
   const float2* wldw;
   const float2* sdw;     // n x 2V pairs (eps * t)
   const float2* qdw;     // n x V pairs
@@ -413,7 +416,7 @@ struct AdjArgs {
   const double* xadd;  // n x V added to the transpose product before the stage
                        // combination (the viscosity source's part), or null
   // double-word gathers (2D Euler, FP64 form): weights on the reverse layout as pairs
-  const float2* wdw[2];
+  const float4* wxydw;
   const float2* whdw;
   const float2* lamdw;  // M2 lam as pairs (set by launch_adj_dw)
 };
