@@ -1010,27 +1010,36 @@ void eval_rhs(mft_ctx* c, double* us, float* us32, double t, const Epilogue& ep_
   // forward gather kernels (FP64-bound, they leave memory and issue slots free) run here;
   // the viscosity kernel waits for it.
   auto rv_norms = [&](cudaStream_t st) {
-    const int mode = (int)c->src_par[iv * 4 + 3];
-    if (c->nseg > 0) {
-      {
-        ProfScope ps(c, MFT_K_MEAN);
-        launch_mean_seg(c->nseg, c->d_seg_off.p, kSegBlocks, V, us, mode, c->seg_partial.p,
-                        c->seg_counter.p, c->seg_mean.p, st);
+    NormArgs na{};
+    na.n = n;
+    na.V = V;
+    na.mode = (int)c->src_par[iv * 4 + 3];
+    na.u = us;
+    na.mean = c->nseg > 0 ? c->seg_mean.p : c->mean.p;
+    na.norms = c->nseg > 0 ? c->seg_norms.p : c->norms.p;
+    na.off = c->nseg > 0 ? c->d_seg_off.p : nullptr;
+    na.nseg = c->nseg;
+    na.partial = c->red_partial.p;
+    na.counter = c->red_counter.p;
+    na.nblocks = c->red_blocks;
+    if (c->nseg > 0 || n <= kNormClusterMax) {
+      if (!c->prof_on) {
+        launch_norms_cluster(na, 3, st);
+      } else {
+        {
+          ProfScope ps(c, MFT_K_MEAN);
+          launch_norms_cluster(na, 1, st);
+        }
+        ProfScope ps(c, MFT_K_LEXMAX);
+        launch_norms_cluster(na, 2, st);
       }
-      ProfScope ps(c, MFT_K_LEXMAX);
-      launch_lexmax_seg(c->nseg, c->d_seg_off.p, kSegBlocks, V, us, c->seg_mean.p, mode,
-                        c->seg_partial.p, c->seg_counter.p + c->nseg, c->seg_norms.p, st,
-                        !c->prof_on);
     } else {
-      const double denom = mode == 0 ? (double)n * V : (double)n;
       {
         ProfScope ps(c, MFT_K_MEAN);
-        launch_mean(n, V, us, denom, c->red_partial.p, c->red_counter.p, c->mean.p,
-                    c->red_blocks, st);
+        launch_norm_sums(na, st);
       }
       ProfScope ps(c, MFT_K_LEXMAX);
-      launch_lexmax(n, V, us, c->mean.p, mode, c->red_partial.p, c->red_counter.p + 1,
-                    c->norms.p, c->red_blocks, st, !c->prof_on);
+      launch_norm_lexmax(na, !c->prof_on, st);
     }
   };
   // With the viscosity formed in the double-word forward gather's epilogue, the norms run
@@ -1834,9 +1843,6 @@ mft_status mft_set_segments(mft_ctx* c, int nseg, const int64_t* offsets, const 
     c->d_seg_off.upload(c->seg_off, s);
     c->d_seg_id.upload(sid, s);
     c->d_seg_h.upload(h, nseg, s);
-    c->seg_partial.alloc((size_t)nseg * kSegBlocks * 8);
-    c->seg_counter.alloc((size_t)2 * nseg);
-    c->seg_counter.zero(s);
     c->seg_mean.alloc((size_t)nseg * 8);
     c->seg_norms.alloc((size_t)nseg * 8);
     MFT_CUDA(cudaStreamSynchronize(s));

@@ -13,6 +13,7 @@
 //   rev        transpose gather -sum_d D_d' s_d (and lap' q) over the reverse
 //              adjacency (hyperviscosity.jl:401-407, :121-134), BC pass 2 and the
 //              SSP-RK stage combination as epilogue.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 #include <math.h>
 
@@ -317,15 +318,56 @@ __device__ double block_sum_lanes(const double* v) {
   return r;
 }
 
+// |x| as a bit pattern: the sign bit cleared (fabs, without an FP64 instruction)
+typedef unsigned long long u64;
+constexpr u64 kAbsMask = 0x7FFFFFFFFFFFFFFFull;
+__device__ __forceinline__ u64 abs_key(double x) { return (u64)__double_as_longlong(x) & kAbsMask; }
+// The pattern of x as an unsigned integer that orders like the value (NaN beyond the
+// infinities on its sign's side), and back.
+__device__ __forceinline__ u64 order_key(double x) {
+  const u64 b = (u64)__double_as_longlong(x);
+  return b ^ ((b >> 63) ? ~0ull : 1ull << 63);
+}
+__device__ __forceinline__ double order_value(u64 k) {
+  return __longlong_as_double((long long)(k ^ ((k >> 63) ? 1ull << 63 : ~0ull)));
+}
+__device__ __forceinline__ u64 warp_max_u64(u64 k) {
+  const unsigned hi = (unsigned)(k >> 32), mh = __reduce_max_sync(kFull, hi);
+  return ((u64)mh << 32) | __reduce_max_sync(kFull, hi == mh ? (unsigned)k : 0u);
+}
+// The block's maximum of k, in every thread.
+__device__ __forceinline__ u64 block_max_u64(u64 k) {
+  __shared__ u64 sh[kWarps];
+  k = warp_max_u64(k);
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = k;
+  __syncthreads();
+  k = sh[0];
+#pragma unroll
+  for (int w = 1; w < kWarps; ++w) k = sh[w] > k ? sh[w] : k;
+  __syncthreads();
+  return k;
+}
+// The first component's part of a lexicographic maximum of |u - mean| over nodes whose first
+// component lies in [lo, hi]: u - m rounds monotonically, so the largest |u - m| is that of an
+// end.
+__device__ __forceinline__ u64 extreme_key(u64 lo, u64 hi, double m) {
+  const u64 a = abs_key(dsub(order_value(lo), m)), b = abs_key(dsub(order_value(hi), m));
+  return a > b ? a : b;
+}
+
 // Sum of u per variable; the last block to finish reduces the block partials in a fixed
 // order (deterministic) and writes mean = sum / denom.  A grid launched after this one
-// with launch_k(pdl) may start at once (it waits for the means with pdl_wait).
-template <int V, bool VEC>
+// with launch_k(pdl) may start at once (it waits for the means with pdl_wait).  EXT: also
+// each block's extremes of the first component (order keys, ext[2 b], ext[2 b + 1]) and, with
+// the mean known, the largest |u_0 - mean_0| of all nodes (top), for k_lexmax.
+template <int V, bool VEC, bool EXT>
 __global__ void __launch_bounds__(kBlock) k_mean(int64_t n, const double* __restrict__ u,
                                                  double denom, double* partial,
-                                                 unsigned* counter, double* mean) {
+                                                 unsigned* counter, double* mean, u64* ext,
+                                                 u64* top) {
   pdl_trigger();
   double acc[V];
+  u64 nlo = 0, hi = 0;  // the complement of the lowest order key, and the highest
 #pragma unroll
   for (int k = 0; k < V; ++k) acc[k] = 0.0;
   // unrolled so that four nodes' loads are in flight together; the additions keep the
@@ -333,14 +375,29 @@ __global__ void __launch_bounds__(kBlock) k_mean(int64_t n, const double* __rest
 #pragma unroll 4
   for (int64_t i = blockIdx.x * (int64_t)kBlock + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * kBlock) {
+    double uv[V];
     if (VEC && V == 4) {
       const double2* u2 = reinterpret_cast<const double2*>(u) + i * 2;
       const double2 a = __ldg(u2), b = __ldg(u2 + 1);
-      acc[0] = dadd(acc[0], a.x); acc[1 % V] = dadd(acc[1 % V], a.y);
-      acc[2 % V] = dadd(acc[2 % V], b.x); acc[3 % V] = dadd(acc[3 % V], b.y);
+      uv[0] = a.x; uv[1 % V] = a.y; uv[2 % V] = b.x; uv[3 % V] = b.y;
     } else {
 #pragma unroll
-      for (int k = 0; k < V; ++k) acc[k] = dadd(acc[k], u[i * V + k]);
+      for (int k = 0; k < V; ++k) uv[k] = u[i * V + k];
+    }
+#pragma unroll
+    for (int k = 0; k < V; ++k) acc[k] = dadd(acc[k], uv[k]);
+    if (EXT) {
+      const u64 x = order_key(uv[0]);
+      hi = x > hi ? x : hi;
+      nlo = ~x > nlo ? ~x : nlo;
+    }
+  }
+  if (EXT) {
+    hi = block_max_u64(hi);
+    nlo = block_max_u64(nlo);
+    if (threadIdx.x == 0) {
+      ext[2 * blockIdx.x] = ~nlo;
+      ext[2 * blockIdx.x + 1] = hi;
     }
   }
   const double tot = block_sum_lanes<V>(acc);
@@ -365,8 +422,22 @@ __global__ void __launch_bounds__(kBlock) k_mean(int64_t n, const double* __rest
 #pragma unroll
     for (int k = 0; k < V; ++k) acc[k] = dadd(acc[k], __ldcg(partial + b * V + k));
   const double all = block_sum_lanes<V>(acc);
-  if (threadIdx.x < V) mean[threadIdx.x] = all / denom;
+  __shared__ double m0;
+  if (threadIdx.x < V) {
+    const double m = all / denom;
+    mean[threadIdx.x] = m;
+    if (threadIdx.x == 0) m0 = m;
+  }
   if (threadIdx.x == 0) *counter = 0u;
+  if (!EXT) return;
+  __syncthreads();
+  u64 best = 0;
+  for (unsigned b = threadIdx.x; b < gridDim.x; b += kBlock) {
+    const u64 x = extreme_key(__ldcg(ext + 2 * b), __ldcg(ext + 2 * b + 1), m0);
+    best = x > best ? x : best;
+  }
+  best = block_max_u64(best);
+  if (threadIdx.x == 0) *top = best;
 }
 
 // ode_maximum(|u - mean|) (mpi.jl:61-81): lexicographic Base.isless order on vectors
@@ -374,9 +445,6 @@ __global__ void __launch_bounds__(kBlock) k_mean(int64_t n, const double* __rest
 // hyperviscosity.jl:310-311).  |u - mean| >= 0, so the IEEE bit pattern of every
 // component orders like its value (NaN above +Inf, as Base.isless does): the maximum
 // is taken on 64-bit integer keys.
-typedef unsigned long long u64;
-// |x| as a bit pattern: the sign bit cleared (fabs, without an FP64 instruction)
-constexpr u64 kAbsMask = 0x7FFFFFFFFFFFFFFFull;
 
 template <int V>
 __device__ __forceinline__ bool key_less(const u64* a, const u64* b) {
@@ -448,41 +516,65 @@ __device__ __forceinline__ void write_norms(const u64* best, double* norms) {
   }
 }
 
+// One node's key against the running maximum; mode 0 forms the later components only where the
+// first one reaches the maximum's.
+template <int V>
+__device__ __forceinline__ void take_node(const double* uv, const double* m, int max_mode,
+                                          u64* best) {
+  u64 x[V];
+  x[0] = abs_key(dsub(uv[0], m[0]));
+  if (max_mode == 0 && x[0] < best[0]) return;
+#pragma unroll
+  for (int k = 1; k < V; ++k) x[k] = abs_key(dsub(uv[k], m[k]));
+  key_max_into<V>(best, x, max_mode);
+}
+
+// Lexicographic maximum (max_mode 0): only the blocks whose extremes (ext, k_mean) reach the
+// largest first component *top read their nodes again -- one or two of them unless many nodes
+// share an extreme; the others finish at once.  Per component (1): every block.  The whole pass
+// read and subtracted everything before: 31 us at 1M nodes between two events, 17 us now (an
+// empty launch takes about 8 so).
 template <int V, bool VEC>
 __global__ void __launch_bounds__(kBlock) k_lexmax(int64_t n, const double* __restrict__ u,
                                                    const double* __restrict__ mean, int max_mode,
                                                    double* partial, unsigned* counter,
-                                                   double* norms) {
+                                                   double* norms, const u64* ext, const u64* top) {
   pdl_trigger();
   pdl_wait();  // the means (k_mean, which this grid may overlap)
   double m[V];
   u64 best[V];
 #pragma unroll
   for (int k = 0; k < V; ++k) { m[k] = __ldcg(mean + k); best[k] = 0ull; }
-  // Threads without nodes keep the all-zero key, the smallest possible: it can only
-  // tie with a real all-zero vector, which has the same value.
-#pragma unroll 4
-  for (int64_t i = blockIdx.x * (int64_t)kBlock + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * kBlock) {
-    double uv[V];
-    if (VEC && V == 4) {
-      const double2* u2 = reinterpret_cast<const double2*>(u) + i * 2;
-      const double2 a = __ldg(u2), b = __ldg(u2 + 1);
-      uv[0] = a.x; uv[1 % V] = a.y; uv[2 % V] = b.x; uv[3 % V] = b.y;
-    } else {
-#pragma unroll
-      for (int k = 0; k < V; ++k) uv[k] = u[i * V + k];
-    }
-    u64 x[V];
-#pragma unroll
-    for (int k = 0; k < V; ++k) x[k] = (u64)__double_as_longlong(dsub(uv[k], m[k])) & kAbsMask;
-    key_max_into<V>(best, x, max_mode);
-  }
-  block_keymax<V>(best, max_mode);
+  const u64 t0 = max_mode == 0 ? __ldcg(top) : 0ull;
+  auto reaches = [&](unsigned b) {
+    return max_mode != 0 || extreme_key(__ldcg(ext + 2 * b), __ldcg(ext + 2 * b + 1), m[0]) == t0;
+  };
   __shared__ int last;
-  if (threadIdx.x == 0) {
+  if (reaches(blockIdx.x)) {
+    // Threads without nodes keep the all-zero key, the smallest possible: it can only
+    // tie with a real all-zero vector, which has the same value.
+    best[0] = t0;
+#pragma unroll 4
+    for (int64_t i = blockIdx.x * (int64_t)kBlock + threadIdx.x; i < n;
+         i += (int64_t)gridDim.x * kBlock) {
+      double uv[V];
+      if (VEC && V == 4) {
+        const double2* u2 = reinterpret_cast<const double2*>(u) + i * 2;
+        const double2 a = __ldg(u2), b = __ldg(u2 + 1);
+        uv[0] = a.x; uv[1 % V] = a.y; uv[2 % V] = b.x; uv[3 % V] = b.y;
+      } else {
 #pragma unroll
-    for (int k = 0; k < V; ++k) partial[blockIdx.x * V + k] = __longlong_as_double((long long)best[k]);
+        for (int k = 0; k < V; ++k) uv[k] = u[i * V + k];
+      }
+      take_node<V>(uv, m, max_mode, best);
+    }
+    block_keymax<V>(best, max_mode);
+    if (threadIdx.x == 0)
+#pragma unroll
+      for (int k = 0; k < V; ++k)
+        partial[blockIdx.x * V + k] = __longlong_as_double((long long)best[k]);
+  }
+  if (threadIdx.x == 0) {
     __threadfence();
     last = (atomicAdd(counter, 1u) == gridDim.x - 1);
   }
@@ -492,6 +584,7 @@ __global__ void __launch_bounds__(kBlock) k_lexmax(int64_t n, const double* __re
 #pragma unroll
   for (int k = 0; k < V; ++k) best[k] = 0ull;
   for (unsigned b = threadIdx.x; b < gridDim.x; b += kBlock) {
+    if (!reaches(b)) continue;
     u64 c[V];
 #pragma unroll
     for (int k = 0; k < V; ++k) c[k] = (u64)__double_as_longlong(__ldcg(partial + b * V + k));
@@ -502,96 +595,110 @@ __global__ void __launch_bounds__(kBlock) k_lexmax(int64_t n, const double* __re
   if (threadIdx.x == 0) *counter = 0u;
 }
 
-// Segmented versions for ensembles: segment s owns nodes [off[s], off[s+1]) and is
-// reduced by `per` blocks (blockIdx.x = s * per + part); the last block of a segment
-// finishes it in the same fixed order as above.
+// The means and norms of small problems and of ensemble members: one cluster of kNormCluster
+// blocks per segment [off[s], off[s+1]) (off null: one segment of n nodes), whose totals meet in
+// distributed shared memory -- one launch and two cluster barriers instead of two grid
+// reductions with their last-block tails.  phases: 1 the means, 2 the norms from the means in
+// memory, 3 both (the same bits).  One rhs! of 2,116 nodes: 85 -> 68 us, 48 SSP-RK3 stages of
+// 16 ensemble members: 5.96 -> 4.93 ms.
+constexpr int kNormCluster = 8;
+constexpr int kNormThreads = 512;
 template <int V>
-__global__ void __launch_bounds__(kBlock) k_mean_seg(const int64_t* __restrict__ off, int per,
-                                                     const double* __restrict__ u, int mode,
-                                                     double* partial, unsigned* counter,
-                                                     double* mean) {
+__global__ void __launch_bounds__(kNormThreads) k_norms_cluster(
+    const int64_t* __restrict__ off, int64_t n, const double* __restrict__ u, int mode,
+    double* mean, double* norms, int phases) {
   pdl_trigger();
-  const int sg = blockIdx.x / per, part = blockIdx.x % per;
-  const int64_t lo = off[sg], hi = off[sg + 1];
-  double acc[V];
+  constexpr int NW = kNormThreads / 32;
+  __shared__ double sums[V][NW], total[V], mean_s[V];
+  __shared__ u64 keys[NW][V], key[V];
+  auto cluster = cooperative_groups::this_cluster();
+  const int sg = blockIdx.x / kNormCluster, rank = (int)cluster.block_rank();
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int64_t lo = off ? off[sg] : 0, hi = off ? off[sg + 1] : n;
+  const int64_t first = lo + rank * kNormThreads + threadIdx.x;
+  constexpr int64_t step = (int64_t)kNormCluster * kNormThreads;
+  auto node = [&](int64_t i, double* uv) {
+    if (V == 4) {
+      const double2* u2 = reinterpret_cast<const double2*>(u) + i * 2;
+      const double2 a = __ldg(u2), b = __ldg(u2 + 1);
+      uv[0] = a.x; uv[1 % V] = a.y; uv[2 % V] = b.x; uv[3 % V] = b.y;
+    } else {
+      uv[0] = u[i];
+    }
+  };
+  if (phases & 1) {
+    double acc[V];
 #pragma unroll
-  for (int k = 0; k < V; ++k) acc[k] = 0.0;
-  for (int64_t i = lo + (int64_t)part * kBlock + threadIdx.x; i < hi; i += (int64_t)per * kBlock) {
+    for (int k = 0; k < V; ++k) acc[k] = 0.0;
+#pragma unroll 4
+    for (int64_t i = first; i < hi; i += step) {
+      double uv[V];
+      node(i, uv);
 #pragma unroll
-    for (int k = 0; k < V; ++k) acc[k] = dadd(acc[k], u[i * V + k]);
+      for (int k = 0; k < V; ++k) acc[k] = dadd(acc[k], uv[k]);
+    }
+    const double x = warp_sum_scatter<V>(acc, lane);
+    if ((lane & (V == 4 ? 7 : 31)) == 0) sums[V == 4 ? lane >> 3 : 0][wid] = x;
+    __syncthreads();
+    if (wid < V) {
+      double t = lane < NW ? sums[wid][lane] : 0.0;
+#pragma unroll
+      for (int o = NW / 2; o > 0; o >>= 1) t = dadd(t, __shfl_xor_sync(kFull, t, o));
+      if (lane == 0) total[wid] = t;
+    }
+    cluster.sync();
+    if (threadIdx.x < V) {
+      double t = 0.0;
+      for (int r = 0; r < kNormCluster; ++r)
+        t = dadd(t, *cluster.map_shared_rank(&total[threadIdx.x], r));
+      const double denom = mode == 0 ? (double)(hi - lo) * V : (double)(hi - lo);
+      mean_s[threadIdx.x] = t / denom;
+      if (rank == 0) mean[sg * V + threadIdx.x] = mean_s[threadIdx.x];
+    }
+  } else if (threadIdx.x < V) {
+    mean_s[threadIdx.x] = mean[sg * V + threadIdx.x];
   }
-  const double tot = block_sum_lanes<V>(acc);
-  __shared__ int last;
-  if (threadIdx.x < 32) {
-    double t[V];
+  __syncthreads();
+  if (phases & 2) {
+    double m[V];
+    u64 best[V];
 #pragma unroll
-    for (int k = 0; k < V; ++k) t[k] = __shfl_sync(kFull, tot, k);
-    if (threadIdx.x == 0) {
+    for (int k = 0; k < V; ++k) { m[k] = mean_s[k]; best[k] = 0ull; }
+#pragma unroll 4
+    for (int64_t i = first; i < hi; i += step) {
+      double uv[V];
+      node(i, uv);
+      take_node<V>(uv, m, mode, best);
+    }
+    auto fold = [&](int from) {
+      for (int o = from; o > 0; o >>= 1) {
+        u64 c[V];
 #pragma unroll
-      for (int k = 0; k < V; ++k) partial[blockIdx.x * V + k] = t[k];
-      __threadfence();
-      last = (atomicAdd(counter + sg, 1u) == (unsigned)per - 1);
+        for (int k = 0; k < V; ++k) c[k] = __shfl_xor_sync(kFull, best[k], o);
+        key_max_into<V>(best, c, mode);
+      }
+    };
+    fold(16);
+    if (lane == 0)
+#pragma unroll
+      for (int k = 0; k < V; ++k) keys[wid][k] = best[k];
+    __syncthreads();
+    if (wid == 0) {
+#pragma unroll
+      for (int k = 0; k < V; ++k) best[k] = lane < NW ? keys[lane][k] : 0ull;
+      fold(NW / 2);
+      if (lane < V) key[lane] = lane == 0 ? best[0] : lane == 1 ? best[1 % V] : lane == 2 ? best[2 % V] : best[3 % V];
+    }
+    cluster.sync();
+    if (rank == 0 && wid == 0) {
+#pragma unroll
+      for (int k = 0; k < V; ++k)
+        best[k] = lane < kNormCluster ? *cluster.map_shared_rank(&key[k], lane) : 0ull;
+      fold(kNormCluster / 2);
+      write_norms<V>(best, norms + sg * 2 * V);
     }
   }
-  __syncthreads();
-  if (!last) return;
-  __threadfence();
-#pragma unroll
-  for (int k = 0; k < V; ++k) acc[k] = 0.0;
-  for (int b = threadIdx.x; b < per; b += kBlock)
-#pragma unroll
-    for (int k = 0; k < V; ++k) acc[k] = dadd(acc[k], __ldcg(partial + (sg * per + b) * V + k));
-  const double all = block_sum_lanes<V>(acc);
-  if (threadIdx.x < V) {
-    const double denom = mode == 0 ? (double)(hi - lo) * V : (double)(hi - lo);
-    mean[sg * V + threadIdx.x] = all / denom;
-  }
-  if (threadIdx.x == 0) counter[sg] = 0u;
-}
-
-template <int V>
-__global__ void __launch_bounds__(kBlock) k_lexmax_seg(const int64_t* __restrict__ off, int per,
-                                                       const double* __restrict__ u,
-                                                       const double* __restrict__ mean,
-                                                       int max_mode, double* partial,
-                                                       unsigned* counter, double* norms) {
-  pdl_trigger();
-  pdl_wait();  // the means (k_mean_seg)
-  const int sg = blockIdx.x / per, part = blockIdx.x % per;
-  const int64_t lo = off[sg], hi = off[sg + 1];
-  double m[V];
-  u64 best[V];
-#pragma unroll
-  for (int k = 0; k < V; ++k) { m[k] = __ldcg(mean + sg * V + k); best[k] = 0ull; }
-  for (int64_t i = lo + (int64_t)part * kBlock + threadIdx.x; i < hi; i += (int64_t)per * kBlock) {
-    u64 x[V];
-#pragma unroll
-    for (int k = 0; k < V; ++k) x[k] = (u64)__double_as_longlong(dsub(u[i * V + k], m[k])) & kAbsMask;
-    key_max_into<V>(best, x, max_mode);
-  }
-  block_keymax<V>(best, max_mode);
-  __shared__ int last;
-  if (threadIdx.x == 0) {
-#pragma unroll
-    for (int k = 0; k < V; ++k) partial[blockIdx.x * V + k] = __longlong_as_double((long long)best[k]);
-    __threadfence();
-    last = (atomicAdd(counter + sg, 1u) == (unsigned)per - 1);
-  }
-  __syncthreads();
-  if (!last) return;
-  __threadfence();
-#pragma unroll
-  for (int k = 0; k < V; ++k) best[k] = 0ull;
-  for (int b = threadIdx.x; b < per; b += kBlock) {
-    u64 c[V];
-#pragma unroll
-    for (int k = 0; k < V; ++k)
-      c[k] = (u64)__double_as_longlong(__ldcg(partial + (sg * per + b) * V + k));
-    key_max_into<V>(best, c, max_mode);
-  }
-  block_keymax<V>(best, max_mode);
-  if (threadIdx.x < 32) write_norms<V>(best, norms + sg * 2 * V);
-  if (threadIdx.x == 0) counter[sg] = 0u;
+  cluster.sync();  // no block leaves while another reads its shared memory
 }
 
 // ------------------------------------------------------------------ viscosity
@@ -884,45 +991,52 @@ void launch_fwd_f64(const FwdArgs& a, cudaStream_t s) {
 void launch_mean(int64_t n, int V, const double* u, double denom, double* partial,
                  unsigned* counter, double* mean, int nblocks, cudaStream_t s) {
   const bool vec = (reinterpret_cast<uintptr_t>(u) & 15) == 0;
-  if (V == 4 && vec) k_mean<4, true><<<nblocks, kBlock, 0, s>>>(n, u, denom, partial, counter, mean);
-  else if (V == 4) k_mean<4, false><<<nblocks, kBlock, 0, s>>>(n, u, denom, partial, counter, mean);
-  else k_mean<1, false><<<nblocks, kBlock, 0, s>>>(n, u, denom, partial, counter, mean);
-  MFT_LAUNCH_CHECK();
-}
-
-void launch_lexmax(int64_t n, int V, const double* u, const double* mean, int max_mode,
-                   double* partial, unsigned* counter, double* norms, int nblocks,
-                   cudaStream_t s, bool pdl) {
-  const bool vec = (reinterpret_cast<uintptr_t>(u) & 15) == 0;
   if (V == 4 && vec)
-    launch_k(k_lexmax<4, true>, nblocks, kBlock, 0, s, pdl, n, u, mean, max_mode, partial,
-             counter, norms);
+    k_mean<4, true, false><<<nblocks, kBlock, 0, s>>>(n, u, denom, partial, counter, mean, nullptr, nullptr);
   else if (V == 4)
-    launch_k(k_lexmax<4, false>, nblocks, kBlock, 0, s, pdl, n, u, mean, max_mode, partial,
-             counter, norms);
+    k_mean<4, false, false><<<nblocks, kBlock, 0, s>>>(n, u, denom, partial, counter, mean, nullptr, nullptr);
   else
-    launch_k(k_lexmax<1, false>, nblocks, kBlock, 0, s, pdl, n, u, mean, max_mode, partial,
-             counter, norms);
-}
-
-void launch_mean_seg(int nseg, const int64_t* off, int per, int V, const double* u, int mode,
-                     double* partial, unsigned* counter, double* mean, cudaStream_t s) {
-  if (nseg <= 0) return;
-  if (V == 4) k_mean_seg<4><<<nseg * per, kBlock, 0, s>>>(off, per, u, mode, partial, counter, mean);
-  else k_mean_seg<1><<<nseg * per, kBlock, 0, s>>>(off, per, u, mode, partial, counter, mean);
+    k_mean<1, false, false><<<nblocks, kBlock, 0, s>>>(n, u, denom, partial, counter, mean, nullptr, nullptr);
   MFT_LAUNCH_CHECK();
 }
 
-void launch_lexmax_seg(int nseg, const int64_t* off, int per, int V, const double* u,
-                       const double* mean, int max_mode, double* partial, unsigned* counter,
-                       double* norms, cudaStream_t s, bool pdl) {
-  if (nseg <= 0) return;
-  if (V == 4)
-    launch_k(k_lexmax_seg<4>, nseg * per, kBlock, 0, s, pdl, off, per, u, mean, max_mode,
-             partial, counter, norms);
+void launch_norm_sums(const NormArgs& a, cudaStream_t s) {
+  u64* ext = reinterpret_cast<u64*>(a.partial + (size_t)a.nblocks * 4);
+  u64* top = reinterpret_cast<u64*>(a.mean + 4);
+  const double denom = a.mode == 0 ? (double)a.n * a.V : (double)a.n;
+  if (a.V == 4)
+    k_mean<4, true, true><<<a.nblocks, kBlock, 0, s>>>(a.n, a.u, denom, a.partial, a.counter, a.mean, ext, top);
   else
-    launch_k(k_lexmax_seg<1>, nseg * per, kBlock, 0, s, pdl, off, per, u, mean, max_mode,
-             partial, counter, norms);
+    k_mean<1, false, true><<<a.nblocks, kBlock, 0, s>>>(a.n, a.u, denom, a.partial, a.counter, a.mean, ext, top);
+  MFT_LAUNCH_CHECK();
+}
+
+void launch_norm_lexmax(const NormArgs& a, bool pdl, cudaStream_t s) {
+  const u64* ext = reinterpret_cast<const u64*>(a.partial + (size_t)a.nblocks * 4);
+  const u64* top = reinterpret_cast<const u64*>(a.mean + 4);
+  if (a.V == 4)
+    launch_k(k_lexmax<4, true>, a.nblocks, kBlock, 0, s, pdl, a.n, a.u, (const double*)a.mean,
+             a.mode, a.partial, a.counter + 1, a.norms, ext, top);
+  else
+    launch_k(k_lexmax<1, false>, a.nblocks, kBlock, 0, s, pdl, a.n, a.u, (const double*)a.mean,
+             a.mode, a.partial, a.counter + 1, a.norms, ext, top);
+}
+
+void launch_norms_cluster(const NormArgs& a, int phases, cudaStream_t s) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = (unsigned)((a.off ? a.nseg : 1) * kNormCluster);
+  cfg.blockDim = kNormThreads;
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = kNormCluster;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  if (a.V == 4)
+    MFT_CUDA(cudaLaunchKernelEx(&cfg, k_norms_cluster<4>, a.off, a.n, a.u, a.mode, a.mean, a.norms, phases));
+  else
+    MFT_CUDA(cudaLaunchKernelEx(&cfg, k_norms_cluster<1>, a.off, a.n, a.u, a.mode, a.mean, a.norms, phases));
 }
 
 void prepare_eps(EpsArgs& a) {

@@ -16,8 +16,6 @@ constexpr int kSlotHv = 4;
 constexpr int kSlots = 5;
 // Threads per block of the node-parallel kernels (sizes the per-block reduction partials).
 constexpr int kBlockHost = 128;
-// Blocks per ensemble member in the segmented reductions.
-constexpr int kSegBlocks = 8;
 
 struct mft_ctx {
   int device = 0;
@@ -131,8 +129,7 @@ struct mft_ctx {
   std::vector<int64_t> seg_off;
   mft::DBuf<int64_t> d_seg_off;
   mft::DBuf<int> d_seg_id;
-  mft::DBuf<double> d_seg_h, seg_partial, seg_mean, seg_norms;
-  mft::DBuf<unsigned> seg_counter;
+  mft::DBuf<double> d_seg_h, seg_mean, seg_norms;
 
   // IGR source work buffers and CG scalars
   mft::DBuf<double> igr_prim, igr_rinv, igr_x, igr_r, igr_u0, igr_u1, igr_c, igr_t, igr_add,

@@ -331,20 +331,37 @@ bool dw_fwd_fuses(int variant);
 float2 gm1_pair(double gamma);
 void launch_fwd_f32(const FwdArgs& a, cudaStream_t s);
 
-// Reductions for the residual viscosity normalisation (last-block-done pattern).
+// Sums of u per variable divided by denom (last-block-done pattern).
 void launch_mean(int64_t n, int V, const double* u, double denom, double* partial,
                  unsigned* counter, double* mean, int nblocks, cudaStream_t s);
-// pdl: launched as a programmatic dependent of the k_mean launch just before it
-void launch_lexmax(int64_t n, int V, const double* u, const double* mean, int max_mode,
-                   double* partial, unsigned* counter, double* norms, int nblocks,
-                   cudaStream_t s, bool pdl = false);
+
+// The residual viscosity's normalisation: means (ode_mean) and norms (ode_maximum of
+// |u - mean|, then their reciprocals) of u (n x V, 16-byte aligned), mode as mean_mode.
+struct NormArgs {
+  int64_t n;
+  int V, mode;
+  const double* u;
+  double* mean;       // V values (per segment) and, for one problem, one more at [4]
+  double* norms;      // 2 V per segment
+  const int64_t* off; // ensembles: nseg + 1 offsets; null: one problem
+  int nseg;
+  double* partial;    // one problem: 8 nblocks
+  unsigned* counter;  // one problem: 2
+  int nblocks;
+};
+// One problem, two grid reductions: the sums, then the maximum (pdl: launched as a programmatic
+// dependent of the sums just before it).
+void launch_norm_sums(const NormArgs& a, cudaStream_t s);
+void launch_norm_lexmax(const NormArgs& a, bool pdl, cudaStream_t s);
+// Both by one cluster of blocks per segment: phases 1 the means, 2 the norms, 3 both.
+// One problem of at most kNormClusterMax nodes, and ensembles (whose members had eight blocks
+// each before, as many as the cluster).  The cluster's FP64 additions run on eight SMs only, the
+// two grid reductions cost a launch and two last-block tails; one rhs! with the grid reductions /
+// the cluster: 4,096 nodes 78 / 51 us, 32,761: 76 / 71, 65,536: 97 / 86, 131,044: 122 / 146.
+constexpr int64_t kNormClusterMax = 65536;
+void launch_norms_cluster(const NormArgs& a, int phases, cudaStream_t s);
 
 void launch_eps(const EpsArgs& a, cudaStream_t s);
-void launch_mean_seg(int nseg, const int64_t* off, int per, int V, const double* u, int mode,
-                     double* partial, unsigned* counter, double* mean, cudaStream_t s);
-void launch_lexmax_seg(int nseg, const int64_t* off, int per, int V, const double* u,
-                       const double* mean, int max_mode, double* partial, unsigned* counter,
-                       double* norms, cudaStream_t s, bool pdl = false);
 void launch_eps_f32(const EpsArgs& a, cudaStream_t s);
 
 struct RevArgs {
