@@ -890,12 +890,12 @@ static void check_kernel_errors(mft_ctx* c) {
 // Work buffers of the IGR source.
 static void ensure_igr(mft_ctx* c) {
   const size_t n = (size_t)c->n;
-  c->igr_prim.alloc(n * 3);
+  c->igr_prim.alloc(n * 4);
   for (auto* b : {&c->igr_rinv, &c->igr_x, &c->igr_r, &c->igr_u0, &c->igr_u1, &c->igr_c})
     b->alloc(n);
   c->igr_t.alloc(n * 2);
   c->igr_add.alloc(n * 2);
-  c->igr_partial.alloc((n + kBlockHost - 1) / kBlockHost + 1);
+  c->igr_partial.alloc((n + kBlockHost - 1) / kBlockHost + 512);
   if (!c->igr_counter.p) {
     c->igr_counter.alloc(1);
     c->igr_counter.zero(c->stream);
@@ -1067,6 +1067,7 @@ void eval_rhs(mft_ctx* c, double* us, float* us32, double t, const Epilogue& ep_
     ia.ell = c->fwd.view();
     ia.wx = c->fw[0].p;
     ia.wy = c->fw[1].p;
+    ia.wxydw = dw ? reinterpret_cast<const float4*>(c->fwdw[0].p) : nullptr;
     ia.alpha = c->src_par[ig * 4];
     ia.maxiter = (int)c->src_par[ig * 4 + 1];
     ia.prim = c->igr_prim.p;
