@@ -128,7 +128,7 @@ static void spread_quarter(int nrows, const std::vector<int32_t>* lists,
 // each: distinct columns ascending, and each element's position among them), and with
 // spread the rows of the staged groups take their entries in the bank-spreading order of
 // spread_quarter (else, and in the other groups, in structure order).
-void build_ell(int64_t n, const std::vector<int64_t>& rowptr, const std::vector<int32_t>& cols,
+void build_ell(int64_t n, const std::vector<int64_t>& rowptr, const mft::HostVec<int32_t>& cols,
                EllBuf& ell, std::vector<int64_t>& pos, cudaStream_t s, int window = 0,
                const std::vector<int32_t>* base = nullptr, int halo_rows = 0,
                bool spread = false) {
@@ -362,6 +362,55 @@ std::vector<int32_t> morton_order(int dim, int64_t n, const std::vector<double>&
 
 namespace mft {
 
+// The copies go through two pinned blocks: while one arrives, all host threads move the other to
+// its place.  A plain copy into pageable memory ran on one thread, which also took the page
+// faults of freshly allocated arrays.  With the uninitialised host arrays (HostVec) and the
+// neighbour search's buckets built on the device, neighbours and weights of 262,144 nodes with
+// all their outputs: 123 -> 67 ms (blocks of 1 to 32 MB: 66.5 to 69.1).
+constexpr size_t kStageBytes = 4u << 20;
+void copy_out(mft_ctx* c, void* dst, const void* dev, size_t bytes, void* dst2) {
+  cudaStream_t s = c->stream;
+  if (bytes < kStageBytes / 4) {
+    MFT_CUDA(cudaMemcpyAsync(dst, dev, bytes, cudaMemcpyDeviceToHost, s));
+    MFT_CUDA(cudaStreamSynchronize(s));
+    if (dst2) memcpy(dst2, dst, bytes);
+    return;
+  }
+  if (!c->h_stage) {
+    for (auto& e : c->ev_stage)
+      if (!e) MFT_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    if (cudaMallocHost(reinterpret_cast<void**>(&c->h_stage), 2 * kStageBytes) != cudaSuccess) {
+      cudaGetLastError();
+      c->h_stage = nullptr;
+      throw Error(MFT_ERR_NOMEM, "cudaMallocHost of the staging blocks failed");
+    }
+  }
+  const size_t nblk = (bytes + kStageBytes - 1) / kStageBytes;
+  auto size_of = [&](size_t b) { return std::min(kStageBytes, bytes - b * kStageBytes); };
+  auto request = [&](size_t b) {
+    MFT_CUDA(cudaMemcpyAsync(c->h_stage + (b & 1) * kStageBytes,
+                             static_cast<const unsigned char*>(dev) + b * kStageBytes, size_of(b),
+                             cudaMemcpyDeviceToHost, s));
+    MFT_CUDA(cudaEventRecord(c->ev_stage[b & 1], s));
+  };
+  request(0);
+  for (size_t b = 0; b < nblk; ++b) {
+    if (b + 1 < nblk) request(b + 1);
+    MFT_CUDA(cudaEventSynchronize(c->ev_stage[b & 1]));
+    const unsigned char* from = c->h_stage + (b & 1) * kStageBytes;
+    unsigned char* to = static_cast<unsigned char*>(dst) + b * kStageBytes;
+    unsigned char* to2 = dst2 ? static_cast<unsigned char*>(dst2) + b * kStageBytes : nullptr;
+    constexpr size_t kPiece = 128u << 10;
+    const size_t m = size_of(b);
+#pragma omp parallel for schedule(static)
+    for (int64_t p = 0; p < (int64_t)((m + kPiece - 1) / kPiece); ++p) {
+      const size_t o = (size_t)p * kPiece, len = std::min(kPiece, m - o);
+      memcpy(to + o, from + o, len);
+      if (to2) memcpy(to2 + o, from + o, len);
+    }
+  }
+}
+
 static cudaEvent_t pool_event(mft_ctx* c) {
   if (!c->ev_pool.empty()) {
     cudaEvent_t e = c->ev_pool.back();
@@ -419,8 +468,8 @@ void finish_pattern(mft_ctx* c) {
 #pragma omp parallel for schedule(static)
   for (int64_t e = 0; e < nnz; ++e) __atomic_fetch_add(&cp[ci[e] + 1], (int64_t)1, __ATOMIC_RELAXED);
   for (int64_t j = 0; j < n; ++j) cp[j + 1] += cp[j];
-  c->ri.assign(nnz, 0);
-  c->csc2csr.assign(nnz, 0);
+  c->ri.resize(nnz);
+  c->csc2csr.resize(nnz);
   std::vector<int64_t> fill(c->cp.begin(), c->cp.end() - 1);
   int32_t* ri = c->ri.data();
   int64_t* c2r = c->csc2csr.data();
@@ -459,8 +508,8 @@ void finish_pattern(mft_ctx* c) {
 void pattern_from_stencils(mft_ctx* c) {
   const int64_t n = c->n;
   c->rp.assign(n + 1, 0);
-  c->ci.assign(c->st_ci.size(), 0);
-  c->st2csr.assign(c->st_ci.size(), 0);
+  c->ci.resize(c->st_ci.size());
+  c->st2csr.resize(c->st_ci.size());
   // rows sorted by column on all host threads; (column, position) packed in one integer
   // gives one plain sort per row with equal columns in position order (rejected)
   int64_t dup = INT64_MAX;  // smallest row that lists a node twice
@@ -609,7 +658,7 @@ void ensure_device_ops(mft_ctx* c) {
       c->fwdw[k].release(); c->rwdw[k].release();
       continue;
     }
-    const std::vector<double>& v = c->val[k];
+    const HostVec<double>& v = c->val[k];
     d_v.upload(v, s);
     c->fw[k].alloc(c->fwd.n_elems);
     c->rw[k].alloc(c->rev.n_elems);
@@ -1452,6 +1501,9 @@ mft_status mft_ctx_destroy(mft_ctx* c) {
   for (auto e : c->ev_pool) cudaEventDestroy(e);
   for (auto g : c->gexec)
     if (g) cudaGraphExecDestroy(g);
+  if (c->h_stage) cudaFreeHost(c->h_stage);
+  for (auto e : c->ev_stage)
+    if (e) cudaEventDestroy(e);
   for (auto e : c->region_ev)
     if (e) cudaEventDestroy(e);
   delete c;
@@ -1506,6 +1558,7 @@ mft_status mft_set_stencils(mft_ctx* c, const int64_t* rowptr, const int32_t* co
       MFT_REQUIRE(cols[e] >= 0 && cols[e] < c->n, MFT_ERR_ARG, "stencil index out of range");
     c->st_rp.assign(rowptr, rowptr + c->n + 1);
     c->st_ci.assign(cols, cols + nnz);
+    c->d_st_ci.release();
     c->have_stencils = true;
     pattern_from_stencils(c);
   });
@@ -1517,17 +1570,12 @@ mft_status mft_knn(mft_ctx* c, int k, int32_t* out_idx, double* out_dist, double
     MFT_REQUIRE(c->n > 0, MFT_ERR_STATE, "call mft_set_points first");
     MFT_REQUIRE(k >= 1 && k <= c->n && k <= 1024, MFT_ERR_ARG, "k out of range");
     set_device(c);
-    std::vector<int32_t> idx;
-    std::vector<double> dist;
     double dmin = 0, davg = 0;
-    knn_device(c, k, idx, out_dist ? &dist : nullptr, &dmin, &davg);
+    knn_device(c, k, out_idx, out_dist, &dmin, &davg);
     c->st_rp.resize(c->n + 1);
     for (int64_t i = 0; i <= c->n; ++i) c->st_rp[i] = i * k;
-    c->st_ci = idx;
     c->have_stencils = true;
     pattern_from_stencils(c);
-    if (out_idx) memcpy(out_idx, idx.data(), idx.size() * sizeof(int32_t));
-    if (out_dist) memcpy(out_dist, dist.data(), dist.size() * sizeof(double));
     if (out_dx_min) *out_dx_min = dmin;
     if (out_dx_avg) *out_dx_avg = davg;
   });
@@ -1550,26 +1598,32 @@ mft_status mft_weights(mft_ctx* c, int op, int rbf_pow, int polydeg, int deriv_o
     MFT_REQUIRE(polydeg >= 0 && polydeg <= 6, MFT_ERR_ARG, "polydeg out of range");
     MFT_REQUIRE(rbf_pow >= 1 && rbf_pow <= 15, MFT_ERR_ARG, "rbf_pow out of range");
     set_device(c);
-    std::vector<double> w;
-    weights_device(c, rbf_pow, polydeg, deriv_order, w, out_max_resid);
     const int64_t nnz = (int64_t)c->st_ci.size();
     const int D = c->dim;
-    if (out_w) memcpy(out_w, w.data(), (size_t)nnz * D * sizeof(double));
+    HostVec<double> own;
+    if (!out_w) own.resize((size_t)nnz * D);
+    double* w = out_w ? out_w : own.data();
+    weights_device(c, rbf_pow, polydeg, deriv_order, w, out_max_resid);
+    const int64_t* to = c->st2csr.data();
     if (op == MFT_OP_GRAD) {
+      double* v[3] = {nullptr, nullptr, nullptr};
       for (int d = 0; d < D; ++d) {
-        c->val[d].assign(nnz, 0.0);
-        double* vd = c->val[d].data();
-#pragma omp parallel for schedule(static)
-        for (int64_t e = 0; e < nnz; ++e) vd[c->st2csr[e]] = w[e * D + d];
+        c->val[d].resize(nnz);
+        v[d] = c->val[d].data();
         c->have_val[d] = true;
       }
+#pragma omp parallel for schedule(static)
+      for (int64_t e = 0; e < nnz; ++e)
+        for (int d = 0; d < D; ++d) v[d][to[e]] = w[e * D + d];
     } else {
       const int slot = op == MFT_OP_LAP ? kSlotLap : kSlotHv;
-      c->val[slot].assign(nnz, 0.0);
+      c->val[slot].resize(nnz);
+      double* v = c->val[slot].data();
+#pragma omp parallel for schedule(static)
       for (int64_t e = 0; e < nnz; ++e) {
         double acc = w[e * D];
         for (int d = 1; d < D; ++d) acc = acc + w[e * D + d];  // sum(operators)
-        c->val[slot][c->st2csr[e]] = acc;
+        v[to[e]] = acc;
       }
       c->have_val[slot] = true;
     }
@@ -1607,7 +1661,7 @@ mft_status mft_load_csc(mft_ctx* c, int op, int comp, int64_t n, const int64_t* 
       c->rp.assign(n + 1, 0);
       for (int64_t p = 0; p < nnz; ++p) c->rp[rowval[p]]++;
       for (int64_t i = 0; i < n; ++i) c->rp[i + 1] += c->rp[i];
-      c->ci.assign(nnz, 0);
+      c->ci.resize(nnz);
       std::vector<int64_t> fill(c->rp.begin(), c->rp.end() - 1);
       for (int64_t j = 0; j < n; ++j)
         for (int64_t p = colptr[j] - 1; p < colptr[j + 1] - 1; ++p)
@@ -1620,7 +1674,7 @@ mft_status mft_load_csc(mft_ctx* c, int op, int comp, int64_t n, const int64_t* 
       c->have_stencils = false;
     }
     const int slot = op == MFT_OP_GRAD ? comp : (op == MFT_OP_LAP ? kSlotLap : kSlotHv);
-    c->val[slot].assign(nnz, 0.0);
+    c->val[slot].resize(nnz);
     for (int64_t p = 0; p < nnz; ++p) c->val[slot][c->csc2csr[p]] = nzval[p];
     c->have_val[slot] = true;
     c->dev_dirty = true;

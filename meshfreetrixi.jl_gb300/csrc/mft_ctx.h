@@ -32,18 +32,19 @@ struct mft_ctx {
 
   // stencils in caller order (centre first)
   std::vector<int64_t> st_rp;
-  std::vector<int32_t> st_ci;
+  mft::HostVec<int32_t> st_ci;
+  mft::DBuf<int32_t> d_st_ci;  // the same on the device after mft_knn (empty: upload st_ci)
   bool have_stencils = false;
 
   // operator pattern: CSR rows with ascending columns, its CSC view, and maps
   bool have_pattern = false;
   std::vector<int64_t> rp;
-  std::vector<int32_t> ci;
+  mft::HostVec<int32_t> ci;
   std::vector<int64_t> cp;
-  std::vector<int32_t> ri;
-  std::vector<int64_t> csc2csr;  // CSC entry -> CSR entry
-  std::vector<int64_t> st2csr;   // stencil entry -> CSR entry (when built from stencils)
-  std::vector<double> val[kSlots];
+  mft::HostVec<int32_t> ri;
+  mft::HostVec<int64_t> csc2csr;  // CSC entry -> CSR entry
+  mft::HostVec<int64_t> st2csr;   // stencil entry -> CSR entry (when built from stencils)
+  mft::HostVec<double> val[kSlots];
   bool have_val[kSlots] = {false, false, false, false, false};
   bool dev_dirty = true;
   mft::EllBuf fwd, rev;
@@ -164,6 +165,8 @@ struct mft_ctx {
   mft::StepParams* h_tab = nullptr;  // pinned staging of the step table
   size_t h_tab_n = 0;
   cudaEvent_t ev_tab = nullptr;      // the last table copy
+  unsigned char* h_stage = nullptr;  // pinned staging of copy_out
+  cudaEvent_t ev_stage[2] = {nullptr, nullptr};
   int* h_kerr = nullptr;             // pinned copy of the device error word
   mft::DBuf<int> d_ctr;
 
@@ -225,10 +228,15 @@ void pattern_from_stencils(mft_ctx* c);
 // Reverse CSC view + ELL/maps rebuild flags after the CSR pattern is set.
 void finish_pattern(mft_ctx* c);
 // KNN and weights (mft_knn.cu, mft_weights.cu)
-void knn_device(mft_ctx* c, int k, std::vector<int32_t>& idx, std::vector<double>* dist,
-                double* dx_min, double* dx_avg);
-void weights_device(mft_ctx* c, int rbf_pow, int polydeg, int deriv_order,
-                    std::vector<double>& w_out, double* max_resid);
+// knn_device: the stencils into c->st_ci (kept on the device in c->d_st_ci) and, where given,
+// out_idx; the distances into dist (n k) where given.  weights_device: st_ci.size() dim values
+// into w.
+void knn_device(mft_ctx* c, int k, int32_t* out_idx, double* dist, double* dx_min, double* dx_avg);
+void weights_device(mft_ctx* c, int rbf_pow, int polydeg, int deriv_order, double* w,
+                    double* max_resid);
+// Device memory into pageable host memory (dst, and dst2 when not null), behind the work queued
+// on the context's stream; returns when the bytes are there.
+void copy_out(mft_ctx* c, void* dst, const void* dev, size_t bytes, void* dst2 = nullptr);
 void weights_batch(mft_ctx* c, int ngroups, const mft_weight_group* groups, double* max_resid);
 // The viscosity source's part of the adjoint of rhs! (mft_adjoint_visc.cu).
 void visc_adjoint_terms(mft_ctx* c, const double* u_bc, const double* lam, double* out);

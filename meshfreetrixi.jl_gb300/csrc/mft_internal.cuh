@@ -4,8 +4,11 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <memory>
+#include <new>
 #include <stdexcept>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "meshfree_gb300.h"
@@ -58,6 +61,29 @@ inline void launch_k(void (*k)(KArgs...), dim3 grid, dim3 block, size_t smem, cu
   MFT_CUDA(cudaLaunchKernelEx(&cfg, k, args...));
 }
 
+// Host array whose resize leaves new elements uninitialised: the large per-entry arrays are
+// filled by all host threads at once, and a zero fill by one thread before that touched every
+// page first (690 MB of them in the set-up of 262,144 nodes).
+template <class T>
+struct NoInit {
+  using value_type = T;
+  NoInit() = default;
+  template <class U>
+  NoInit(const NoInit<U>&) {}
+  T* allocate(size_t n) { return std::allocator<T>().allocate(n); }
+  void deallocate(T* p, size_t n) { std::allocator<T>().deallocate(p, n); }
+  template <class U>
+  void construct(U* p) { ::new (static_cast<void*>(p)) U; }
+  template <class U, class... A>
+  void construct(U* p, A&&... a) { ::new (static_cast<void*>(p)) U(std::forward<A>(a)...); }
+  template <class U>
+  bool operator==(const NoInit<U>&) const { return true; }
+  template <class U>
+  bool operator!=(const NoInit<U>&) const { return false; }
+};
+template <class T>
+using HostVec = std::vector<T, NoInit<T>>;
+
 // Owning device buffer (cudaMalloc / cudaFree).
 template <class T>
 struct DBuf {
@@ -88,7 +114,8 @@ struct DBuf {
     alloc(count);
     if (count) MFT_CUDA(cudaMemcpyAsync(p, h, count * sizeof(T), cudaMemcpyHostToDevice, s));
   }
-  void upload(const std::vector<T>& h, cudaStream_t s) { upload(h.data(), h.size(), s); }
+  template <class A>
+  void upload(const std::vector<T, A>& h, cudaStream_t s) { upload(h.data(), h.size(), s); }
   void zero(cudaStream_t s) {
     if (n) MFT_CUDA(cudaMemsetAsync(p, 0, n * sizeof(T), s));
   }

@@ -183,6 +183,103 @@ __global__ void __launch_bounds__(kKnnBlock) k_knn(KnnArgs a) {
   }
 }
 
+// Buckets on the device: the cell of every node and the cells' counts, their prefix sum (one
+// block), and the nodes placed cell by cell.  The order inside a cell is whatever the atomics
+// give; the search result does not depend on it.
+struct BinArgs {
+  int dim;
+  int64_t n, ncell;
+  int64_t nc[3];
+  double lo[3], cs[3];
+  const double* xyz;
+  int32_t* cell;
+  int* count;       // ncell, zero on entry; the fill cursors after the scan
+  int64_t* cstart;  // ncell + 1
+  int32_t* cpts;
+  double* cxyz;
+};
+__global__ void k_bin_count(BinArgs a) {
+  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (i >= a.n) return;
+  int64_t cc = 0, mul = 1;
+  for (int d = 0; d < a.dim; ++d) {
+    int64_t ci = (int64_t)floor(__ddiv_rn(__dsub_rn(a.xyz[i * a.dim + d], a.lo[d]), a.cs[d]));
+    ci = ci < 0 ? 0 : ci > a.nc[d] - 1 ? a.nc[d] - 1 : ci;
+    cc += ci * mul;
+    mul *= a.nc[d];
+  }
+  a.cell[i] = (int32_t)cc;
+  atomicAdd(a.count + cc, 1);
+}
+__global__ void __launch_bounds__(1024) k_bin_scan(BinArgs a) {
+  __shared__ int warp_sum[32];
+  __shared__ int64_t carry;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  if (threadIdx.x == 0) carry = 0;
+  __syncthreads();
+  constexpr int K = 8;  // cells per thread and round
+  for (int64_t c0 = 0; c0 < a.ncell; c0 += 1024 * K) {
+    const int64_t c = c0 + (int64_t)threadIdx.x * K;
+    int v[K], t = 0;
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      v[k] = c + k < a.ncell ? a.count[c + k] : 0;
+      t += v[k];
+    }
+    int x = t;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= o) x += y;
+    }
+    if (lane == 31) warp_sum[wid] = x;
+    __syncthreads();
+    if (wid == 0) {
+      int w = warp_sum[lane];
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, w, o);
+        if (lane >= o) w += y;
+      }
+      warp_sum[lane] = w;
+    }
+    __syncthreads();
+    int64_t at = carry + (wid ? warp_sum[wid - 1] : 0) + x - t;
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      if (c + k < a.ncell) {
+        a.cstart[c + k] = at;
+        a.count[c + k] = (int)at;
+      }
+      at += v[k];
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) carry += warp_sum[31];
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) a.cstart[a.ncell] = carry;
+}
+__global__ void k_bin_fill(BinArgs a) {
+  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (i >= a.n) return;
+  const int64_t p = atomicAdd(a.count + a.cell[i], 1);
+  a.cpts[p] = (int32_t)i;
+  for (int d = 0; d < a.dim; ++d) a.cxyz[p * a.dim + d] = a.xyz[i * a.dim + d];
+}
+// The distances from the squared ones in place (where asked for), and every node's nearest other
+// node's (column 1).
+__global__ void k_dist(int64_t n, int k, double* d2, int all, double* near) {
+  const int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (all) {
+    if (e >= n * k) return;
+    const double d = sqrt(d2[e]);
+    d2[e] = d;
+    if (e % k == 1) near[e / k] = d;
+  } else if (e < n) {
+    near[e] = sqrt(d2[e * k + 1]);
+  }
+}
+
 // Julia's pairwise reduction (Base.mapreduce_impl, block size 1024).
 double pairwise(const double* x, int64_t lo, int64_t hi) {
   if (lo == hi) return x[lo];
@@ -211,18 +308,20 @@ double julia_sum(const std::vector<double>& x) {
 
 }  // namespace
 
-void knn_device(mft_ctx* c, int k, std::vector<int32_t>& idx, std::vector<double>* dist,
-                double* dx_min, double* dx_avg) {
+void knn_device(mft_ctx* c, int k, int32_t* out_idx, double* dist, double* dx_min, double* dx_avg) {
   const int dim = c->dim;
   const int64_t n = c->n;
   const double* x = c->xyz.data();
   double lo[3] = {0, 0, 0}, hi[3] = {0, 0, 0};
   for (int d = 0; d < dim; ++d) {
-    lo[d] = hi[d] = x[d];
+    double l = x[d], h = x[d];
+#pragma omp parallel for schedule(static) reduction(min : l) reduction(max : h)
     for (int64_t i = 1; i < n; ++i) {
-      lo[d] = std::min(lo[d], x[i * dim + d]);
-      hi[d] = std::max(hi[d], x[i * dim + d]);
+      l = std::min(l, x[i * dim + d]);
+      h = std::max(h, x[i * dim + d]);
     }
+    lo[d] = l;
+    hi[d] = h;
   }
   double vol = 1.0;
   for (int d = 0; d < dim; ++d) {
@@ -242,39 +341,40 @@ void knn_device(mft_ctx* c, int k, std::vector<int32_t>& idx, std::vector<double
     if (!c->periodic) cs[d] *= (1.0 + 1e-12);
   }
   const int64_t ncell = nc[0] * nc[1] * nc[2];
-  std::vector<int32_t> cell(n);
-  std::vector<int64_t> cstart(ncell + 1, 0);
-  for (int64_t i = 0; i < n; ++i) {
-    int64_t cc = 0, mul = 1;
-    for (int d = 0; d < dim; ++d) {
-      int64_t ci = (int64_t)floor((x[i * dim + d] - lo[d]) / cs[d]);
-      ci = std::max<int64_t>(0, std::min<int64_t>(ci, nc[d] - 1));
-      cc += ci * mul;
-      mul *= nc[d];
-    }
-    cell[i] = (int32_t)cc;
-    cstart[cc + 1]++;
-  }
-  for (int64_t q = 0; q < ncell; ++q) cstart[q + 1] += cstart[q];
-  std::vector<int32_t> cpts(n);
-  std::vector<double> cxyz((size_t)n * dim);
-  {
-    std::vector<int64_t> fill(cstart.begin(), cstart.end() - 1);
-    for (int64_t i = 0; i < n; ++i) {
-      const int64_t p = fill[cell[i]]++;
-      cpts[p] = (int32_t)i;
-      for (int d = 0; d < dim; ++d) cxyz[p * dim + d] = x[i * dim + d];
-    }
-  }
   cudaStream_t s = c->stream;
-  DBuf<double> d_cxyz, d_d2;
-  DBuf<int32_t> d_cpts, d_cell, d_idx;
+  DBuf<double> d_cxyz, d_d2, d_near;
+  DBuf<int32_t> d_cpts, d_cell;
   DBuf<int64_t> d_cstart;
-  DBuf<int> d_err;
-  d_cxyz.upload(cxyz, s);
-  d_cpts.upload(cpts, s);
-  d_cell.upload(cell, s);
-  d_cstart.upload(cstart, s);
+  DBuf<int> d_err, d_count;
+  d_cxyz.alloc((size_t)n * dim);
+  d_cpts.alloc(n);
+  d_cell.alloc(n);
+  d_cstart.alloc(ncell + 1);
+  d_count.alloc(ncell);
+  d_count.zero(s);
+  BinArgs b{};
+  b.dim = dim;
+  b.n = n;
+  b.ncell = ncell;
+  for (int d = 0; d < 3; ++d) {
+    b.nc[d] = nc[d];
+    b.lo[d] = lo[d];
+    b.cs[d] = cs[d];
+  }
+  b.xyz = c->d_xyz.p;
+  b.cell = d_cell.p;
+  b.count = d_count.p;
+  b.cstart = d_cstart.p;
+  b.cpts = d_cpts.p;
+  b.cxyz = d_cxyz.p;
+  const unsigned gn = (unsigned)((n + 255) / 256);
+  k_bin_count<<<gn, 256, 0, s>>>(b);
+  MFT_LAUNCH_CHECK();
+  k_bin_scan<<<1, 1024, 0, s>>>(b);
+  MFT_LAUNCH_CHECK();
+  k_bin_fill<<<gn, 256, 0, s>>>(b);
+  MFT_LAUNCH_CHECK();
+  DBuf<int32_t> d_idx;
   d_idx.alloc((size_t)n * k);
   d_d2.alloc((size_t)n * k);
   d_err.alloc(1);
@@ -305,35 +405,30 @@ void knn_device(mft_ctx* c, int k, std::vector<int32_t>& idx, std::vector<double
   k_knn<<<(unsigned)((n + kKnnBlock - 1) / kKnnBlock), kKnnBlock, shmem, s>>>(a);
   MFT_LAUNCH_CHECK();
   int err = 0;
-  idx.resize((size_t)n * k);
   MFT_CUDA(cudaMemcpyAsync(&err, d_err.p, sizeof(int), cudaMemcpyDeviceToHost, s));
-  MFT_CUDA(cudaMemcpyAsync(idx.data(), d_idx.p, idx.size() * sizeof(int32_t),
-                           cudaMemcpyDeviceToHost, s));
-  // the squared distances: all of them when asked for, else only the nearest other
-  // node's (column 1, for dx_min / dx_avg)
-  std::vector<double> d2(dist ? (size_t)n * k : (size_t)n);
-  if (dist) {
-    MFT_CUDA(cudaMemcpyAsync(d2.data(), d_d2.p, d2.size() * sizeof(double),
-                             cudaMemcpyDeviceToHost, s));
-  } else if (k >= 2) {
-    MFT_CUDA(cudaMemcpy2DAsync(d2.data(), sizeof(double), d_d2.p + 1, (size_t)k * sizeof(double),
-                               sizeof(double), (size_t)n, cudaMemcpyDeviceToHost, s));
+  if (k >= 2) {
+    d_near.alloc(n);
+    const int64_t m = dist ? n * k : n;
+    k_dist<<<(unsigned)((m + 255) / 256), 256, 0, s>>>(n, k, d_d2.p, dist ? 1 : 0, d_near.p);
+    MFT_LAUNCH_CHECK();
   }
   MFT_CUDA(cudaStreamSynchronize(s));
   MFT_REQUIRE(err == 0, MFT_ERR_ARG, "KNN search could not collect k neighbours");
+  std::swap(c->d_st_ci.p, d_idx.p);
+  std::swap(c->d_st_ci.n, d_idx.n);
+  c->st_ci.resize((size_t)n * k);
+  copy_out(c, c->st_ci.data(), c->d_st_ci.p, c->st_ci.size() * sizeof(int32_t), out_idx);
   if (dist) {
-    dist->resize(d2.size());
-    for (size_t e = 0; e < d2.size(); ++e) (*dist)[e] = sqrt(d2[e]);
+    if (k >= 2) copy_out(c, dist, d_d2.p, (size_t)n * k * sizeof(double));
+    else std::fill(dist, dist + n, 0.0);  // the node itself
   }
-  const int64_t d2_stride = dist ? k : 1, d2_col = dist ? 1 : 0;
   // dx_min = minimum(dists)[2], dx_avg = mean(dists)[2] over the 2-NN query.
   if (k >= 2) {
     std::vector<double> nn(n);
+    copy_out(c, nn.data(), d_near.p, n * sizeof(double));
     double m = INFINITY;
-    for (int64_t i = 0; i < n; ++i) {
-      nn[i] = sqrt(d2[(size_t)i * d2_stride + d2_col]);
+    for (int64_t i = 0; i < n; ++i)
       if (nn[i] < m || isnan(nn[i])) m = nn[i];
-    }
     if (dx_min) *dx_min = m;
     if (dx_avg) *dx_avg = julia_sum(nn) / (double)n;
   } else {

@@ -845,7 +845,9 @@ struct HostGroup {
   const double* d_xyz;   // device coordinates (n x dim)
   const int64_t* rowptr; // host, n + 1
   const int32_t* cols;   // host, rowptr[n]
+  const int32_t* d_cols; // the same on the device, or null
   double* w_out;         // host, rowptr[n] x dim
+  bool keep_on_error;    // leave w_out alone when a system is singular
 };
 
 // All groups' systems, largest first, in persistent launches over size buckets of the
@@ -853,7 +855,8 @@ struct HostGroup {
 // memory and occupancy its largest system allows).
 constexpr int kBucketEdges[] = {48, 64, 80, 104};
 
-static void weights_run(cudaStream_t s, const std::vector<HostGroup>& gs, double* max_resid) {
+static void weights_run(mft_ctx* c, const std::vector<HostGroup>& gs, double* max_resid) {
+  cudaStream_t s = c->stream;
   MFT_REQUIRE(!gs.empty() && gs.size() <= (size_t)kMaxGroups, MFT_ERR_ARG,
               "between 1 and 2 weight groups");
   WArgs a{};
@@ -931,11 +934,11 @@ static void weights_run(cudaStream_t s, const std::vector<HostGroup>& gs, double
     const HostGroup& h = gs[g];
     const int64_t nnz = h.rowptr[h.n];
     d_rp[g].upload(h.rowptr, h.n + 1, s);
-    d_ci[g].upload(h.cols, nnz, s);
+    if (!h.d_cols) d_ci[g].upload(h.cols, nnz, s);
     d_w[g].alloc((size_t)nnz * h.dim);
     if (max_resid) d_res[g].alloc(h.n);
     a.g[g].rowptr = d_rp[g].p;
-    a.g[g].cols = d_ci[g].p;
+    a.g[g].cols = h.d_cols ? h.d_cols : d_ci[g].p;
     a.g[g].xyz = h.d_xyz;
     a.g[g].w_out = d_w[g].p;
     a.g[g].resid = max_resid ? d_res[g].p : nullptr;
@@ -976,18 +979,19 @@ static void weights_run(cudaStream_t s, const std::vector<HostGroup>& gs, double
     MFT_LAUNCH_CHECK();
   }
   int bad = big;
+  MFT_CUDA(cudaMemcpyAsync(&bad, d_bad.p, sizeof(int), cudaMemcpyDeviceToHost, s));
+  MFT_CUDA(cudaStreamSynchronize(s));
   std::vector<std::vector<double>> res(gs.size());
   for (size_t g = 0; g < gs.size(); ++g) {
     const HostGroup& h = gs[g];
-    MFT_CUDA(cudaMemcpyAsync(h.w_out, d_w[g].p, (size_t)h.rowptr[h.n] * h.dim * sizeof(double),
-                             cudaMemcpyDeviceToHost, s));
+    if (bad == big || !h.keep_on_error)
+      copy_out(c, h.w_out, d_w[g].p, (size_t)h.rowptr[h.n] * h.dim * sizeof(double));
     if (max_resid) {
       res[g].resize(h.n);
       MFT_CUDA(cudaMemcpyAsync(res[g].data(), d_res[g].p, h.n * sizeof(double),
                                cudaMemcpyDeviceToHost, s));
     }
   }
-  MFT_CUDA(cudaMemcpyAsync(&bad, d_bad.p, sizeof(int), cudaMemcpyDeviceToHost, s));
   MFT_CUDA(cudaStreamSynchronize(s));
   MFT_REQUIRE(bad == big, MFT_ERR_SINGULAR,
               "saddle-point system of node " + std::to_string(bad) + " has an exactly zero pivot");
@@ -999,8 +1003,8 @@ static void weights_run(cudaStream_t s, const std::vector<HostGroup>& gs, double
   }
 }
 
-void weights_device(mft_ctx* c, int rbf_pow, int polydeg, int deriv_order,
-                    std::vector<double>& w_out, double* max_resid) {
+void weights_device(mft_ctx* c, int rbf_pow, int polydeg, int deriv_order, double* w,
+                    double* max_resid) {
   HostGroup h{};
   h.dim = c->dim;
   h.rbf_pow = rbf_pow;
@@ -1011,9 +1015,10 @@ void weights_device(mft_ctx* c, int rbf_pow, int polydeg, int deriv_order,
   h.d_xyz = c->d_xyz.p;
   h.rowptr = c->st_rp.data();
   h.cols = c->st_ci.data();
-  w_out.resize((size_t)c->st_ci.size() * c->dim);
-  h.w_out = w_out.data();
-  weights_run(c->stream, {h}, max_resid);
+  h.d_cols = c->d_st_ci.n == c->st_ci.size() ? c->d_st_ci.p : nullptr;
+  h.w_out = w;
+  h.keep_on_error = true;
+  weights_run(c, {h}, max_resid);
 }
 
 void weights_batch(mft_ctx* c, int ngroups, const mft_weight_group* groups, double* max_resid) {
@@ -1035,6 +1040,8 @@ void weights_batch(mft_ctx* c, int ngroups, const mft_weight_group* groups, doub
     }
     xyz[g].upload(q.xyz, (size_t)q.n * q.dim, c->stream);
     HostGroup& h = hs[g];
+    h.keep_on_error = false;
+    h.d_cols = nullptr;
     h.dim = q.dim;
     h.rbf_pow = q.rbf_pow;
     h.polydeg = q.polydeg;
@@ -1046,7 +1053,7 @@ void weights_batch(mft_ctx* c, int ngroups, const mft_weight_group* groups, doub
     h.cols = q.cols;
     h.w_out = q.w;
   }
-  weights_run(c->stream, hs, max_resid);
+  weights_run(c, hs, max_resid);
 }
 
 }  // namespace mft
