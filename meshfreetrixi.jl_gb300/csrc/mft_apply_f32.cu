@@ -18,8 +18,20 @@ using namespace dev;
 // HALO: one block per row group (ell.halo_rows rows) first stages the group's neighbour
 // states in shared memory (mft_halo.cuh) and reads them from there; groups without a list
 // load them directly.  The sums are the same in the same order either way.
+// The streamed part of a staged row's entry, requested a group of kStagedGroup entries ahead of
+// its use (pipelined_row), with registers capped for kStagedBlocks blocks of 256 rows per SM.
+// Measured at 1M nodes, forward / transpose us: 3 at four blocks 112 / 157, 4 at four 117 / 160, 5
+// at four 132 / 178, 3 at five 144 / 175, 4 at three 125 / 169 (direct loads: 119 / 219, bulk
+// copies 128 / 227).
+struct Streamed32 {
+  int lc;
+  float wx, wy, wl;
+};
+constexpr int kStagedGroup = 3, kStagedBlocks = 4;
+
 template <bool WT, bool WQ, int FLY, bool HALO = false>
-__global__ void __launch_bounds__(HALO ? kHaloRows : kBlock) k_fwd_euler_f32(FwdArgs a) {
+__global__ void __launch_bounds__(HALO ? kHaloRows : kBlock, HALO ? kStagedBlocks : 1)
+    k_fwd_euler_f32(FwdArgs a) {
   const int64_t r = blockIdx.x * (int64_t)(HALO ? (int)blockDim.x : kBlock) + threadIdx.x;
   const float4* __restrict__ U4 = reinterpret_cast<const float4*>(a.u32);
   extern __shared__ float4 hsm[];
@@ -36,26 +48,30 @@ __global__ void __launch_bounds__(HALO ? kHaloRows : kBlock) k_fwd_euler_f32(Fwd
   const float* __restrict__ wlp = a.wl32;
   const float gm1 = a.gm1_32;
   float f[4] = {0, 0, 0, 0}, tx[4] = {0, 0, 0, 0}, ty[4] = {0, 0, 0, 0}, q[4] = {0, 0, 0, 0};
-  auto entry = [&](int64_t p, const float4 uc) {
-    const float wx = __ldg(wxp + p), wy = __ldg(wyp + p);
+  auto entry = [&](float wx, float wy, float wl, const float4 uc) {
     euler_accum_f32<WT>(gm1, uc, wx, wy, f, tx, ty);
     if (WQ || FLY) {
-      const float wl = __ldg(wlp + p);
       q[0] = fmaf(wl, uc.x, q[0]); q[1] = fmaf(wl, uc.y, q[1]);
       q[2] = fmaf(wl, uc.z, q[2]); q[3] = fmaf(wl, uc.w, q[3]);
     }
   };
   if (HALO && staged) {
-#pragma unroll 4
-    for (int j = 0; j < len; ++j) {
-      const int64_t p = base + ((int64_t)j << 5);
-      entry(p, hsm[__ldg(lcol + p)]);
-    }
+    pipelined_row<kStagedGroup, Streamed32>(
+        len,
+        [&](Streamed32& e, int j) {
+          const int64_t p = base + j * 32;
+          e.lc = __ldg(lcol + p);
+          e.wx = __ldg(wxp + p);
+          e.wy = __ldg(wyp + p);
+          e.wl = (WQ || FLY) ? __ldg(wlp + p) : 0.f;
+        },
+        [&](const Streamed32& e) { entry(e.wx, e.wy, e.wl, hsm[e.lc]); });
   } else {
 #pragma unroll 4
     for (int j = 0; j < len; ++j) {
       const int64_t p = base + ((int64_t)j << 5);
-      entry(p, __ldg(U4 + __ldg(col + p)));
+      entry(__ldg(wxp + p), __ldg(wyp + p), (WQ || FLY) ? __ldg(wlp + p) : 0.f,
+            __ldg(U4 + __ldg(col + p)));
     }
   }
   const float hg = a.hg32;
@@ -212,9 +228,13 @@ __global__ void __launch_bounds__(kBlock) k_eps_f32(EpsArgs a) {
 }
 
 // HALO (V = 4 only): staged neighbour records as in k_fwd_euler_f32 -- s = eps t (two
-// chunks) and q (one chunk).
+// chunks) and q (one chunk).  What bounds the direct loop is the latency of the scattered
+// 32- and 16-byte records behind each position's load (1M nodes: 223 us, 3.3 TB/s); the staged
+// one reads them from shared memory and streams 14 bytes per entry.  (As one loop that chose the
+// source per entry it loaded through generic addresses and lost to the direct one.)
 template <int V, bool RV, bool LAP, bool HALO = false>
-__global__ void __launch_bounds__(HALO ? kHaloRows : kBlock) k_rev_f32(RevArgs a) {
+__global__ void __launch_bounds__(HALO ? kHaloRows : kBlock, HALO ? kStagedBlocks : 1)
+    k_rev_f32(RevArgs a) {
   static_assert(!HALO || V == 4, "staged transpose gather: 2D Euler");
   constexpr int NCH = (RV ? 2 : 0) + (LAP ? 1 : 0);
   const int64_t r = blockIdx.x * (int64_t)(HALO ? (int)blockDim.x : kBlock) + threadIdx.x;
@@ -235,26 +255,41 @@ __global__ void __launch_bounds__(HALO ? kHaloRows : kBlock) k_rev_f32(RevArgs a
   float sx[V], sy[V], sl[V];
 #pragma unroll
   for (int v = 0; v < V; ++v) { sx[v] = 0.f; sy[v] = 0.f; sl[v] = 0.f; }
+  auto add4 = [](float* s, float w, float4 x) {
+    s[0] = fmaf(w, x.x, s[0]); s[1 % V] = fmaf(w, x.y, s[1 % V]);
+    s[2 % V] = fmaf(w, x.z, s[2 % V]); s[3 % V] = fmaf(w, x.w, s[3 % V]);
+  };
+  if constexpr (HALO && NCH > 0) {
+    if (staged)
+      pipelined_row<kStagedGroup, Streamed32>(
+          len,
+          [&](Streamed32& e, int j) {
+            const int64_t p = base + j * 32;
+            e.lc = __ldg(a.ell.lcol + p);
+            if (RV) {
+              e.wx = __ldg(a.w32[0] + p);
+              e.wy = __ldg(a.w32[1] + p);
+            }
+            if (LAP) e.wl = __ldg(a.wl32 + p);
+          },
+          [&](const Streamed32& e) {
+            if (RV) {
+              add4(sx, e.wx, hsm[halo_at<NCH>(0, e.lc, hs)]);
+              add4(sy, e.wy, hsm[halo_at<NCH>(1, e.lc, hs)]);
+            }
+            if (LAP) add4(sl, e.wl, hsm[halo_at<NCH>(RV ? 2 : 0, e.lc, hs)]);
+          });
+  }
 #pragma unroll 4
-  for (int j = 0; j < len; ++j) {
+  for (int j = staged ? len : 0; j < len; ++j) {
     const int64_t p = base + ((int64_t)j << 5);
-    const int c = (HALO && staged) ? (int)__ldg(a.ell.lcol + p) : __ldg(a.ell.col + p);
+    const int c = __ldg(a.ell.col + p);
     if (RV) {
       const float wx = __ldg(a.w32[0] + p), wy = __ldg(a.w32[1] + p);
       if (V == 4) {
-        float4 xs, ys;
-        if (HALO && staged) {
-          xs = hsm[halo_at<NCH>(0, c, hs)];
-          ys = hsm[halo_at<NCH>(1, c, hs)];
-        } else {
-          const F8 st = ldg_f8(a.s32 + (int64_t)c * 8);
-          xs = st.lo;
-          ys = st.hi;
-        }
-        sx[0] = fmaf(wx, xs.x, sx[0]); sx[1] = fmaf(wx, xs.y, sx[1]);
-        sx[2] = fmaf(wx, xs.z, sx[2]); sx[3] = fmaf(wx, xs.w, sx[3]);
-        sy[0] = fmaf(wy, ys.x, sy[0]); sy[1] = fmaf(wy, ys.y, sy[1]);
-        sy[2] = fmaf(wy, ys.z, sy[2]); sy[3] = fmaf(wy, ys.w, sy[3]);
+        const F8 st = ldg_f8(a.s32 + (int64_t)c * 8);
+        add4(sx, wx, st.lo);
+        add4(sy, wy, st.hi);
       } else {
         const float2 s2 = __ldg(reinterpret_cast<const float2*>(a.s32) + c);
         sx[0] = fmaf(wx, s2.x, sx[0]);
@@ -263,15 +298,8 @@ __global__ void __launch_bounds__(HALO ? kHaloRows : kBlock) k_rev_f32(RevArgs a
     }
     if (LAP) {
       const float wl = __ldg(a.wl32 + p);
-      if (V == 4) {
-        const float4 qq = (HALO && staged)
-                              ? hsm[halo_at<NCH>(RV ? 2 : 0, c, hs)]
-                              : __ldg(reinterpret_cast<const float4*>(a.q32) + c);
-        sl[0] = fmaf(wl, qq.x, sl[0]); sl[1] = fmaf(wl, qq.y, sl[1]);
-        sl[2] = fmaf(wl, qq.z, sl[2]); sl[3] = fmaf(wl, qq.w, sl[3]);
-      } else {
-        sl[0] = fmaf(wl, __ldg(a.q32 + c), sl[0]);
-      }
+      if (V == 4) add4(sl, wl, __ldg(reinterpret_cast<const float4*>(a.q32) + c));
+      else sl[0] = fmaf(wl, __ldg(a.q32 + c), sl[0]);
     }
   }
   const float hg = a.hg32;
