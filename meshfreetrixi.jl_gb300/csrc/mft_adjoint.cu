@@ -166,27 +166,37 @@ __global__ void __launch_bounds__(kBlock) k_adj_f64(AdjArgs a) {
   adj_finish<V, EULER, BC, HV>(a, i, gx, gy, gh);
 }
 
-// M2 lam as double-word pairs (n x 4 pairs): the cotangent the double-word adjoint
+// M2 lam at node c as double-word chunks.
+template <bool BC>
+static __device__ __forceinline__ void lam_chunks(const double* __restrict__ lam, const BcDev& bc,
+                                                  int64_t c, float4* out) {
+  double l[4];
+  load_row<4>(lam, c, l);
+  if (BC) mask_rows<4>(bc, c, l);
+  out[0] = dw::chunk(dw::split(l[0]), dw::split(l[1]));
+  out[1] = dw::chunk(dw::split(l[2]), dw::split(l[3]));
+}
+
+// M2 lam as double-word chunks (two per node): the cotangent the direct double-word adjoint
 // gather reads, masked once per node instead of once per stencil entry.
 template <bool BC>
 __global__ void k_lam_pairs(int64_t n, const double* __restrict__ lam, BcDev bc,
                             float4* __restrict__ out) {
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= n) return;
-  double l[4];
-  load_row<4>(lam, i, l);
-  if (BC) mask_rows<4>(bc, i, l);
-  const float2 a = dw::split(l[0]), b = dw::split(l[1]), c = dw::split(l[2]),
-               d = dw::split(l[3]);
-  out[i * 2] = dw::chunk(a, b);
-  out[i * 2 + 1] = dw::chunk(c, d);
+  lam_chunks<BC>(lam, bc, i, out + i * 2);
 }
 
 // The adjoint gather of 2D Euler in double-word FP32 arithmetic (as the forward form's
 // gathers; the sums over the reverse adjacency in pairs, the node part in FP64).  HV 0
 // (no hyperviscosity) or 2 (Flyer, whose term gathers the same M2 lam).
-// HALO: blocks of one row group stage the group's neighbour cotangent pairs in shared
-// memory first (mft_halo.cuh); same sums, same order.
+// HALO: blocks of one row group form the group's neighbour cotangents while staging them in
+// shared memory (a group without a list forms them per entry); same sums, same order.  A group's
+// neighbours are 1.8 times its rows, the splits run on the integer pipe, and the kernel that
+// wrote them for every node before is gone (one launch per stage, 65,536 nodes).  With the
+// streamed loads in groups of kAdjGroup ahead the gather took 26.4 us between events against
+// 29.2 (groups of 2 / 3 / 4 / 5: 27.4 / 27.0 / 26.3 / 27.2).
+constexpr int kAdjGroup = 6;
 template <bool BC, int HV, bool HALO>
 __global__ void __launch_bounds__(HALO ? kHaloRows : kBlock) k_adj_dw(AdjArgs a) {
   const int64_t row = blockIdx.x * (int64_t)(HALO ? (int)blockDim.x : kBlock) + threadIdx.x;
@@ -194,7 +204,16 @@ __global__ void __launch_bounds__(HALO ? kHaloRows : kBlock) k_adj_dw(AdjArgs a)
   extern __shared__ float4 hsm[];
   bool staged = false;
   if (HALO) {
-    staged = stage_halo<2>(a.ell, hsm, [&](int k, int64_t c) { return L4 + c * 2 + k; });
+    const int h0 = __ldg(a.ell.halo_off + blockIdx.x);
+    const int nh = __ldg(a.ell.halo_off + blockIdx.x + 1) - h0;
+    for (int q = threadIdx.x; q < nh; q += blockDim.x) {
+      float4 l[2];
+      lam_chunks<BC>(a.lam, a.bc, (int64_t)__ldg(a.ell.halo_col + h0 + q), l);
+      hsm[halo_at<2>(0, q, a.ell.halo_stride)] = l[0];
+      hsm[halo_at<2>(1, q, a.ell.halo_stride)] = l[1];
+    }
+    __syncthreads();
+    staged = nh > 0;
   }
   if (row >= a.n) return;
   const int64_t i = ell_node(a.ell, row);
@@ -204,32 +223,47 @@ __global__ void __launch_bounds__(HALO ? kHaloRows : kBlock) k_adj_dw(AdjArgs a)
   dw::Acc2 gx[2], gy[2], gh[2];
 #pragma unroll
   for (int k = 0; k < 2; ++k) gx[k] = gy[k] = gh[k] = dw::zero2();
-#pragma unroll 2
-  for (int j = 0; j < len; ++j) {
-    const int64_t p = base + ((int64_t)j << 5);
-    const float4 wxy = __ldg(a.wxydw + p);
-    dw::DW2 l[2];
-    if (HALO && staged) {
-      const int lc = __ldg(a.ell.lcol + p);
-      l[0] = dw::pair2(hsm[halo_at<2>(0, lc, hs)]);
-      l[1] = dw::pair2(hsm[halo_at<2>(1, lc, hs)]);
-    } else {
-      const int64_t c = __ldg(a.ell.col + p);
-      l[0] = dw::pair2(__ldg(L4 + c * 2));
-      l[1] = dw::pair2(__ldg(L4 + c * 2 + 1));
-    }
-    const dw::DW2 wx = dw::both(dw::chunk_a(wxy)), wy = dw::both(dw::chunk_b(wxy));
+  struct Streamed {
+    int at;  // the neighbour's place in the group's list, or its node
+    float4 wxy;
+    float2 wh;
+  };
+  auto load = [&](Streamed& e, int j) {
+    const int64_t p = base + j * 32;
+    e.at = HALO && staged ? (int)__ldg(a.ell.lcol + p) : __ldg(a.ell.col + p);
+    e.wxy = __ldg(a.wxydw + p);
+    if (HV == 2) e.wh = __ldg(a.whdw + p);
+  };
+  auto take = [&](const Streamed& e, float4 l0, float4 l1) {
+    const dw::DW2 l[2] = {dw::pair2(l0), dw::pair2(l1)};
+    const dw::DW2 wx = dw::both(dw::chunk_a(e.wxy)), wy = dw::both(dw::chunk_b(e.wxy));
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
       dw::fma_acc2(gx[k], wx, l[k]);
       dw::fma_acc2(gy[k], wy, l[k]);
     }
     if constexpr (HV == 2) {
-      const dw::DW2 wh = dw::both(__ldg(a.whdw + p));
+      const dw::DW2 wh = dw::both(e.wh);
 #pragma unroll
       for (int k = 0; k < 2; ++k) dw::fma_acc2(gh[k], wh, l[k]);
     }
-  }
+  };
+  // a loop for each source of the records: a choice per entry loads through generic addresses
+  if (HALO && staged)
+    pipelined_row<kAdjGroup, Streamed>(len, load, [&](const Streamed& e) {
+      take(e, hsm[halo_at<2>(0, e.at, hs)], hsm[halo_at<2>(1, e.at, hs)]);
+    });
+  else
+    pipelined_row<2, Streamed>(len, load, [&](const Streamed& e) {
+      float4 l[2];
+      if (HALO) {
+        lam_chunks<BC>(a.lam, a.bc, e.at, l);
+      } else {
+        l[0] = __ldg(L4 + (int64_t)e.at * 2);
+        l[1] = __ldg(L4 + (int64_t)e.at * 2 + 1);
+      }
+      take(e, l[0], l[1]);
+    });
   // the Jacobian product in double-word arithmetic from the sums as pairs
   float2 gxp[4], gyp[4];
   double ghd[4];
@@ -310,10 +344,12 @@ void launch_adj_dw(const AdjArgs& a, float2* lam_pairs, bool staged, cudaStream_
   if (a.n <= 0) return;
   MFT_REQUIRE(a.V == 4 && a.eq == MFT_EQ_EULER2D && a.hv != 1, MFT_ERR_UNSUPPORTED,
               "double-word adjoint gather: 2D Euler without Tominec hyperviscosity");
-  const unsigned gn = grid_for(a.n, 256);
-  if (a.has_bc) k_lam_pairs<true><<<gn, 256, 0, s>>>(a.n, a.lam, a.bc, reinterpret_cast<float4*>(lam_pairs));
-  else k_lam_pairs<false><<<gn, 256, 0, s>>>(a.n, a.lam, a.bc, reinterpret_cast<float4*>(lam_pairs));
-  MFT_LAUNCH_CHECK();
+  if (!(staged && a.ell.halo_off)) {
+    const unsigned gn = grid_for(a.n, 256);
+    if (a.has_bc) k_lam_pairs<true><<<gn, 256, 0, s>>>(a.n, a.lam, a.bc, reinterpret_cast<float4*>(lam_pairs));
+    else k_lam_pairs<false><<<gn, 256, 0, s>>>(a.n, a.lam, a.bc, reinterpret_cast<float4*>(lam_pairs));
+    MFT_LAUNCH_CHECK();
+  }
   AdjArgs b = a;
   b.lamdw = lam_pairs;
   if (staged && a.ell.halo_off) {
