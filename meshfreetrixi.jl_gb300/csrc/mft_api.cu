@@ -916,15 +916,25 @@ void launch_rev(mft_ctx* c, const RevArgs& a) {
 // Device error word set by kernels with bounded waits; read at synchronisation points.
 // Synchronises the stream and reads the word: the word's copy into pinned memory is
 // queued behind the work, so one synchronisation covers both.
-static void check_kernel_errors(mft_ctx* c) {
+// Pinned host copy of the error word, mapped for the device.
+static int* host_error_word(mft_ctx* c) {
+  if (!c->h_kerr) {
+    MFT_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&c->h_kerr), sizeof(int), cudaHostAllocMapped));
+    *c->h_kerr = 0;
+  }
+  return c->h_kerr;
+}
+// brought: the call's last kernel has written the word (launch_soa_from_aos).
+static void check_kernel_errors(mft_ctx* c, bool brought = false) {
   if (!c->kerr.p) {
     MFT_CUDA(cudaStreamSynchronize(c->stream));
     return;
   }
-  if (!c->h_kerr) MFT_CUDA(cudaMallocHost(reinterpret_cast<void**>(&c->h_kerr), sizeof(int)));
-  MFT_CUDA(cudaMemcpyAsync(c->h_kerr, c->kerr.p, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+  host_error_word(c);
+  if (!brought)
+    MFT_CUDA(cudaMemcpyAsync(c->h_kerr, c->kerr.p, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
   MFT_CUDA(cudaStreamSynchronize(c->stream));
-  const int e = *c->h_kerr;
+  const int e = *static_cast<volatile int*>(c->h_kerr);
   if (e != 0) {
     c->kerr.zero(c->stream);
     MFT_CUDA(cudaStreamSynchronize(c->stream));
@@ -1933,9 +1943,12 @@ mft_status mft_rhs_device(mft_ctx* c, double* du, double* u, double t) {
     ep.kind = kOutDu;
     ep.out = c->work_du.p;
     eval_rhs(c, c->work_u.p, u32, t, ep);
-    launch_soa_from_aos(c->work_du.p, du, n, V, s);
-    launch_soa_from_aos(c->work_u.p, u, n, V, s);
-    check_kernel_errors(c);
+    // u only changes at listed boundary nodes; the last kernel brings the error word
+    const bool back = c->nb > 0;
+    int* word = host_error_word(c);
+    launch_soa_from_aos(c->work_du.p, du, n, V, s, back ? nullptr : c->kerr.p, word);
+    if (back) launch_soa_from_aos(c->work_u.p, u, n, V, s, c->kerr.p, word);
+    check_kernel_errors(c, true);
   });
 }
 
@@ -1961,13 +1974,16 @@ mft_status mft_rhs(mft_ctx* c, double* const* du, double* const* u, int nvars, d
     ep.kind = kOutDu;
     ep.out = c->work_du.p;
     eval_rhs(c, c->work_u.p, u32, t, ep);
+    // u only changes at listed boundary nodes
+    const bool back = c->nb > 0;
     launch_soa_from_aos(c->work_du.p, c->soa.p, n, V, s);
-    launch_soa_from_aos(c->work_u.p, c->soa2.p, n, V, s);
+    if (back) launch_soa_from_aos(c->work_u.p, c->soa2.p, n, V, s);
     for (int v = 0; v < V; ++v) {
       MFT_CUDA(cudaMemcpyAsync(du[v], c->soa.p + (size_t)v * n, n * sizeof(double),
                                cudaMemcpyDeviceToHost, s));
-      MFT_CUDA(cudaMemcpyAsync(u[v], c->soa2.p + (size_t)v * n, n * sizeof(double),
-                               cudaMemcpyDeviceToHost, s));
+      if (back)
+        MFT_CUDA(cudaMemcpyAsync(u[v], c->soa2.p + (size_t)v * n, n * sizeof(double),
+                                 cudaMemcpyDeviceToHost, s));
     }
     check_kernel_errors(c);
   });
@@ -2947,8 +2963,8 @@ mft_status mft_rhs_adjoint_device(mft_ctx* c, double* out, const double* lam, co
     launch_aos_from_soa(lam, c->adj_lam[0].p, n, V, s);
     eval_rhs_adjoint(c, c->work_u.p, c->adj_lam[0].p, kAdjPlain, 0.0, nullptr, c->adj_lam[1].p,
                      t);
-    launch_soa_from_aos(c->adj_lam[1].p, out, n, V, s);
-    check_kernel_errors(c);
+    launch_soa_from_aos(c->adj_lam[1].p, out, n, V, s, c->kerr.p, host_error_word(c));
+    check_kernel_errors(c, true);
   });
 }
 

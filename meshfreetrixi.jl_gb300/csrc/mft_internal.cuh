@@ -219,7 +219,10 @@ struct Epilogue {
 // (implemented in mft_apply.cu; all enqueue on `s` and return after launch)
 
 void launch_aos_from_soa(const double* soa, double* aos, int64_t n, int V, cudaStream_t s);
-void launch_soa_from_aos(const double* aos, double* soa, int64_t n, int V, cudaStream_t s);
+// err, host_err: also *host_err = *err (host memory mapped for the device): a call's last kernel
+// brings the error word along, without a copy of its own.
+void launch_soa_from_aos(const double* aos, double* soa, int64_t n, int V, cudaStream_t s,
+                         const int* err = nullptr, int* host_err = nullptr);
 void launch_aos_to_f32(const double* aos, float* a32, int64_t count, cudaStream_t s);
 // out[pos[e]] = v[e] (and out32[pos[e]] = (float) v[e] when out32 is not null, and the
 // double-word pair (h, l) of v[e] when outdw is not null): the operator values of structure
