@@ -194,35 +194,23 @@ __global__ void k_lam_pairs(int64_t n, const double* __restrict__ lam, BcDev bc,
 // shared memory (a group without a list forms them per entry); same sums, same order.  A group's
 // neighbours are 1.8 times its rows, the splits run on the integer pipe, and the kernel that
 // wrote them for every node before is gone (one launch per stage, 65,536 nodes).  With the
-// streamed loads in groups of kAdjGroup ahead the gather took 26.4 us between events against
-// 29.2 (groups of 2 / 3 / 4 / 5: 27.4 / 27.0 / 26.3 / 27.2).
+// streamed loads in groups of kAdjGroup ahead the gather and that kernel took 26.4 us between
+// events against 29.2 (groups of 2 / 3 / 4 / 5: 27.4 / 27.0 / 26.3 / 27.2); without that kernel and
+// with the first entries requested before the staging 23.9.
 constexpr int kAdjGroup = 6;
 template <bool BC, int HV, bool HALO>
 __global__ void __launch_bounds__(HALO ? kHaloRows : kBlock) k_adj_dw(AdjArgs a) {
   const int64_t row = blockIdx.x * (int64_t)(HALO ? (int)blockDim.x : kBlock) + threadIdx.x;
   const float4* __restrict__ L4 = reinterpret_cast<const float4*>(a.lamdw);
   extern __shared__ float4 hsm[];
-  bool staged = false;
-  if (HALO) {
-    const int h0 = __ldg(a.ell.halo_off + blockIdx.x);
-    const int nh = __ldg(a.ell.halo_off + blockIdx.x + 1) - h0;
-    for (int q = threadIdx.x; q < nh; q += blockDim.x) {
-      float4 l[2];
-      lam_chunks<BC>(a.lam, a.bc, (int64_t)__ldg(a.ell.halo_col + h0 + q), l);
-      hsm[halo_at<2>(0, q, a.ell.halo_stride)] = l[0];
-      hsm[halo_at<2>(1, q, a.ell.halo_stride)] = l[1];
-    }
-    __syncthreads();
-    staged = nh > 0;
-  }
-  if (row >= a.n) return;
-  const int64_t i = ell_node(a.ell, row);
-  const int64_t base = a.ell.slice_off[row >> 5] + (row & 31);
-  const int len = a.ell.row_len[row];
+  const bool live = row < a.n;
+  const int64_t i = live ? ell_node(a.ell, row) : 0;
+  const int64_t base = live ? a.ell.slice_off[row >> 5] + (row & 31) : 0;
+  const int len = live ? a.ell.row_len[row] : 0;
   const int hs = a.ell.halo_stride;
-  dw::Acc2 gx[2], gy[2], gh[2];
-#pragma unroll
-  for (int k = 0; k < 2; ++k) gx[k] = gy[k] = gh[k] = dw::zero2();
+  const int h0 = HALO ? __ldg(a.ell.halo_off + blockIdx.x) : 0;
+  const int nh = HALO ? __ldg(a.ell.halo_off + blockIdx.x + 1) - h0 : 0;
+  const bool staged = nh > 0;
   struct Streamed {
     int at;  // the neighbour's place in the group's list, or its node
     float4 wxy;
@@ -234,6 +222,21 @@ __global__ void __launch_bounds__(HALO ? kHaloRows : kBlock) k_adj_dw(AdjArgs a)
     e.wxy = __ldg(a.wxydw + p);
     if (HV == 2) e.wh = __ldg(a.whdw + p);
   };
+  Streamed ahead[2][kAdjGroup];
+  if (HALO && staged) {
+    pipelined_open<kAdjGroup>(len, ahead, load);
+    for (int q = threadIdx.x; q < nh; q += blockDim.x) {
+      float4 l[2];
+      lam_chunks<BC>(a.lam, a.bc, (int64_t)__ldg(a.ell.halo_col + h0 + q), l);
+      hsm[halo_at<2>(0, q, hs)] = l[0];
+      hsm[halo_at<2>(1, q, hs)] = l[1];
+    }
+    __syncthreads();
+  }
+  if (!live) return;
+  dw::Acc2 gx[2], gy[2], gh[2];
+#pragma unroll
+  for (int k = 0; k < 2; ++k) gx[k] = gy[k] = gh[k] = dw::zero2();
   auto take = [&](const Streamed& e, float4 l0, float4 l1) {
     const dw::DW2 l[2] = {dw::pair2(l0), dw::pair2(l1)};
     const dw::DW2 wx = dw::both(dw::chunk_a(e.wxy)), wy = dw::both(dw::chunk_b(e.wxy));
@@ -250,7 +253,7 @@ __global__ void __launch_bounds__(HALO ? kHaloRows : kBlock) k_adj_dw(AdjArgs a)
   };
   // a loop for each source of the records: a choice per entry loads through generic addresses
   if (HALO && staged)
-    pipelined_row<kAdjGroup, Streamed>(len, load, [&](const Streamed& e) {
+    pipelined_run<kAdjGroup>(len, ahead, load, [&](const Streamed& e) {
       take(e, hsm[halo_at<2>(0, e.at, hs)], hsm[halo_at<2>(1, e.at, hs)]);
     });
   else

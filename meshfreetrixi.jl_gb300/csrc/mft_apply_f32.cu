@@ -22,7 +22,7 @@ using namespace dev;
 // its use (pipelined_row), with registers capped for kStagedBlocks blocks of 256 rows per SM.
 // Measured at 1M nodes, forward / transpose us: 3 at four blocks 112 / 157, 4 at four 117 / 160, 5
 // at four 132 / 178, 3 at five 144 / 175, 4 at three 125 / 169 (direct loads: 119 / 219, bulk
-// copies 128 / 227).
+// copies 128 / 227); with the first entries requested before the staging 110 / 155.
 struct Streamed32 {
   int lc;
   float wx, wy, wl;
@@ -35,17 +35,30 @@ __global__ void __launch_bounds__(HALO ? kHaloRows : kBlock, HALO ? kStagedBlock
   const int64_t r = blockIdx.x * (int64_t)(HALO ? (int)blockDim.x : kBlock) + threadIdx.x;
   const float4* __restrict__ U4 = reinterpret_cast<const float4*>(a.u32);
   extern __shared__ float4 hsm[];
-  bool staged = false;
-  if (HALO) staged = stage_halo<1>(a.ell, hsm, [&](int, int64_t c) { return U4 + c; });
-  if (r >= a.n) return;
-  const int64_t i = ell_node(a.ell, r);
-  const int64_t base = a.ell.slice_off[r >> 5] + (r & 31);
-  const int len = a.ell.row_len[r];
+  const bool live = r < a.n;
+  const int64_t i = live ? ell_node(a.ell, r) : 0;
+  const int64_t base = live ? a.ell.slice_off[r >> 5] + (r & 31) : 0;
+  const int len = live ? a.ell.row_len[r] : 0;
   const int32_t* __restrict__ col = a.ell.col;
   const uint16_t* __restrict__ lcol = a.ell.lcol;
   const float* __restrict__ wxp = a.w32[0];
   const float* __restrict__ wyp = a.w32[1];
   const float* __restrict__ wlp = a.wl32;
+  Streamed32 ahead[2][kStagedGroup];
+  auto load = [&](Streamed32& e, int j) {
+    const int64_t p = base + j * 32;
+    e.lc = __ldg(lcol + p);
+    e.wx = __ldg(wxp + p);
+    e.wy = __ldg(wyp + p);
+    e.wl = (WQ || FLY) ? __ldg(wlp + p) : 0.f;
+  };
+  bool staged = false;
+  if (HALO) {
+    if (__ldg(a.ell.halo_off + blockIdx.x + 1) > __ldg(a.ell.halo_off + blockIdx.x))
+      pipelined_open<kStagedGroup>(len, ahead, load);
+    staged = stage_halo<1>(a.ell, hsm, [&](int, int64_t c) { return U4 + c; });
+  }
+  if (!live) return;
   const float gm1 = a.gm1_32;
   float f[4] = {0, 0, 0, 0}, tx[4] = {0, 0, 0, 0}, ty[4] = {0, 0, 0, 0}, q[4] = {0, 0, 0, 0};
   auto entry = [&](float wx, float wy, float wl, const float4 uc) {
@@ -56,16 +69,9 @@ __global__ void __launch_bounds__(HALO ? kHaloRows : kBlock, HALO ? kStagedBlock
     }
   };
   if (HALO && staged) {
-    pipelined_row<kStagedGroup, Streamed32>(
-        len,
-        [&](Streamed32& e, int j) {
-          const int64_t p = base + j * 32;
-          e.lc = __ldg(lcol + p);
-          e.wx = __ldg(wxp + p);
-          e.wy = __ldg(wyp + p);
-          e.wl = (WQ || FLY) ? __ldg(wlp + p) : 0.f;
-        },
-        [&](const Streamed32& e) { entry(e.wx, e.wy, e.wl, hsm[e.lc]); });
+    pipelined_run<kStagedGroup>(len, ahead, load, [&](const Streamed32& e) {
+      entry(e.wx, e.wy, e.wl, hsm[e.lc]);
+    });
   } else {
 #pragma unroll 4
     for (int j = 0; j < len; ++j) {
@@ -239,19 +245,32 @@ __global__ void __launch_bounds__(HALO ? kHaloRows : kBlock, HALO ? kStagedBlock
   constexpr int NCH = (RV ? 2 : 0) + (LAP ? 1 : 0);
   const int64_t r = blockIdx.x * (int64_t)(HALO ? (int)blockDim.x : kBlock) + threadIdx.x;
   extern __shared__ float4 hsm[];
+  const bool live = r < a.n;
+  const int64_t i = live ? ell_node(a.ell, r) : 0;
+  const int64_t base = live ? a.ell.slice_off[r >> 5] + (r & 31) : 0;
+  const int len = live ? a.ell.row_len[r] : 0;
+  const int hs = a.ell.halo_stride;
+  Streamed32 ahead[2][kStagedGroup];
+  auto load = [&](Streamed32& e, int j) {
+    const int64_t p = base + j * 32;
+    e.lc = __ldg(a.ell.lcol + p);
+    if (RV) {
+      e.wx = __ldg(a.w32[0] + p);
+      e.wy = __ldg(a.w32[1] + p);
+    }
+    if (LAP) e.wl = __ldg(a.wl32 + p);
+  };
   bool staged = false;
   if (HALO && NCH > 0) {
     const float4* S4 = reinterpret_cast<const float4*>(a.s32);
     const float4* Q4 = reinterpret_cast<const float4*>(a.q32);
+    if (__ldg(a.ell.halo_off + blockIdx.x + 1) > __ldg(a.ell.halo_off + blockIdx.x))
+      pipelined_open<kStagedGroup>(len, ahead, load);
     staged = stage_halo<NCH>(a.ell, hsm, [&](int k, int64_t c) {
       return (RV && k < 2) ? S4 + c * 2 + k : Q4 + c;
     });
   }
-  if (r >= a.n) return;
-  const int64_t i = ell_node(a.ell, r);
-  const int64_t base = a.ell.slice_off[r >> 5] + (r & 31);
-  const int len = a.ell.row_len[r];
-  const int hs = a.ell.halo_stride;
+  if (!live) return;
   float sx[V], sy[V], sl[V];
 #pragma unroll
   for (int v = 0; v < V; ++v) { sx[v] = 0.f; sy[v] = 0.f; sl[v] = 0.f; }
@@ -261,17 +280,7 @@ __global__ void __launch_bounds__(HALO ? kHaloRows : kBlock, HALO ? kStagedBlock
   };
   if constexpr (HALO && NCH > 0) {
     if (staged)
-      pipelined_row<kStagedGroup, Streamed32>(
-          len,
-          [&](Streamed32& e, int j) {
-            const int64_t p = base + j * 32;
-            e.lc = __ldg(a.ell.lcol + p);
-            if (RV) {
-              e.wx = __ldg(a.w32[0] + p);
-              e.wy = __ldg(a.w32[1] + p);
-            }
-            if (LAP) e.wl = __ldg(a.wl32 + p);
-          },
+      pipelined_run<kStagedGroup>(len, ahead, load,
           [&](const Streamed32& e) {
             if (RV) {
               add4(sx, e.wx, hsm[halo_at<NCH>(0, e.lc, hs)]);

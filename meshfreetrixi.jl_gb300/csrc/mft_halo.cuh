@@ -100,30 +100,42 @@ __device__ __forceinline__ bool stage_halo(const EllView& ell, float4* sm, Chunk
 // A staged row's loop with the streamed loads in software pipeline: Entry (positions, weights;
 // load(e, j) requests entry j's) in two register groups of G; a group's loads are issued before
 // the other group is used, so that a group's arithmetic covers their latency.  The entries are
-// used in order, use(e).
-template <int G, typename Entry, typename Load, typename Use>
-__device__ __forceinline__ void pipelined_row(int len, Load load, Use use) {
-  Entry e[2][G];
-  auto get = [&](Entry* x, int g) {
+// used in order, use(e).  pipelined_open requests the first two groups (where the row has them):
+// a kernel does that before it stages its neighbours, whose latency then covers theirs.
+template <int G, typename Entry, typename Load>
+__device__ __forceinline__ void pipelined_get(Entry* x, int g, Load& load) {
 #pragma unroll
-    for (int k = 0; k < G; ++k) load(x[k], g * G + k);
-  };
+  for (int k = 0; k < G; ++k) load(x[k], g * G + k);
+}
+template <int G, typename Entry, typename Load>
+__device__ __forceinline__ void pipelined_open(int len, Entry (&e)[2][G], Load& load) {
   const int ng = len / G;
-  if (ng > 0) get(e[0], 0);
+  if (ng > 0) pipelined_get<G>(e[0], 0, load);
+  if (ng > 1) pipelined_get<G>(e[1], 1, load);
+}
+template <int G, typename Entry, typename Load, typename Use>
+__device__ __forceinline__ void pipelined_run(int len, Entry (&e)[2][G], Load& load, Use use) {
+  const int ng = len / G;
   for (int g = 0; g < ng; g += 2) {
-    if (g + 1 < ng) get(e[1], g + 1);
 #pragma unroll
     for (int k = 0; k < G; ++k) use(e[0][k]);
-    if (g + 2 < ng) get(e[0], g + 2);
+    if (g + 2 < ng) pipelined_get<G>(e[0], g + 2, load);
     if (g + 1 < ng) {
 #pragma unroll
       for (int k = 0; k < G; ++k) use(e[1][k]);
+      if (g + 3 < ng) pipelined_get<G>(e[1], g + 3, load);
     }
   }
   for (int j = ng * G; j < len; ++j) {
     load(e[0][0], j);
     use(e[0][0]);
   }
+}
+template <int G, typename Entry, typename Load, typename Use>
+__device__ __forceinline__ void pipelined_row(int len, Load load, Use use) {
+  Entry e[2][G];
+  pipelined_open<G>(len, e, load);
+  pipelined_run<G>(len, e, load, use);
 }
 
 }  // namespace

@@ -303,8 +303,7 @@ struct IgrStream {
 // group without a list, chunk(c) itself.  What does not depend on the kernel before -- the row,
 // the list, and the first 2 G entries' weights -- is requested before wait(), which returns
 // whether there is anything to do: the weights' latency and the launch then overlap that
-// kernel's tail and the staging.  Two register groups of G entries alternate (as in
-// pipelined_row).  (STAGED: two loops, because one that chose the source per entry loaded
+// kernel's tail and the staging.  (STAGED: two loops, because one that chose the source per entry loaded
 // through generic addresses.)  Every thread of the block must call it.
 template <int G, bool STAGED, typename Wait, typename Chunk, typename Sum>
 __device__ __forceinline__ bool igr_gather_as(const IgrArgs& a, int64_t r, int h0, int nh, float4* sm,
@@ -318,17 +317,11 @@ __device__ __forceinline__ bool igr_gather_as(const IgrArgs& a, int64_t r, int h
     x.lc = STAGED ? (int)__ldg(a.ell.lcol + p) : __ldg(a.ell.col + p);
     x.wxy = __ldg(a.wxydw + p);
   };
-  auto get = [&](IgrStream* x, int g) {
-#pragma unroll
-    for (int k = 0; k < G; ++k) load(x[k], g * G + k);
-  };
   auto use = [&](const IgrStream& x) { sum(x.wxy, STAGED ? sm[x.lc] : chunk((int64_t)x.lc)); };
-  const int ng = len / G;
   const int q0 = threadIdx.x, q1 = q0 + blockDim.x;
   const int c0 = STAGED && q0 < nh ? __ldg(a.ell.halo_col + h0 + q0) : -1;
   const int c1 = STAGED && q1 < nh ? __ldg(a.ell.halo_col + h0 + q1) : -1;
-  if (ng > 0) get(e[0], 0);
-  if (ng > 1) get(e[1], 1);
+  pipelined_open<G>(len, e, load);
   if (!wait()) return false;
   if (STAGED) {
     const float4 v0 = c0 >= 0 ? chunk(c0) : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -339,20 +332,7 @@ __device__ __forceinline__ bool igr_gather_as(const IgrArgs& a, int64_t r, int h
       sm[q] = chunk((int64_t)__ldg(a.ell.halo_col + h0 + q));
     __syncthreads();
   }
-  for (int g = 0; g < ng; g += 2) {
-#pragma unroll
-    for (int k = 0; k < G; ++k) use(e[0][k]);
-    if (g + 2 < ng) get(e[0], g + 2);
-    if (g + 1 < ng) {
-#pragma unroll
-      for (int k = 0; k < G; ++k) use(e[1][k]);
-      if (g + 3 < ng) get(e[1], g + 3);
-    }
-  }
-  for (int j = ng * G; j < len; ++j) {
-    load(e[0][0], j);
-    use(e[0][0]);
-  }
+  pipelined_run<G>(len, e, load, use);
   return true;
 }
 template <int G, typename Wait, typename Chunk, typename Sum>
