@@ -370,20 +370,19 @@ namespace mft {
 constexpr size_t kStageBytes = 4u << 20;
 void copy_out(mft_ctx* c, void* dst, const void* dev, size_t bytes, void* dst2) {
   cudaStream_t s = c->stream;
-  if (bytes < kStageBytes / 4) {
+  if (bytes >= kStageBytes / 4 && !c->h_stage) {
+    for (auto& e : c->ev_stage)
+      if (!e) MFT_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    if (cudaMallocHost(reinterpret_cast<void**>(&c->h_stage), 2 * kStageBytes) != cudaSuccess) {
+      cudaGetLastError();  // no pinned memory to be had: the plain copy below
+      c->h_stage = nullptr;
+    }
+  }
+  if (bytes < kStageBytes / 4 || !c->h_stage) {
     MFT_CUDA(cudaMemcpyAsync(dst, dev, bytes, cudaMemcpyDeviceToHost, s));
     MFT_CUDA(cudaStreamSynchronize(s));
     if (dst2) memcpy(dst2, dst, bytes);
     return;
-  }
-  if (!c->h_stage) {
-    for (auto& e : c->ev_stage)
-      if (!e) MFT_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-    if (cudaMallocHost(reinterpret_cast<void**>(&c->h_stage), 2 * kStageBytes) != cudaSuccess) {
-      cudaGetLastError();
-      c->h_stage = nullptr;
-      throw Error(MFT_ERR_NOMEM, "cudaMallocHost of the staging blocks failed");
-    }
   }
   const size_t nblk = (bytes + kStageBytes - 1) / kStageBytes;
   auto size_of = [&](size_t b) { return std::min(kStageBytes, bytes - b * kStageBytes); };
