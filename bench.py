@@ -101,8 +101,8 @@ def parse():
     ap.add_argument("--riemann-side", type=int, default=1024,
                     help="nodes per side of the Riemann FP32/FP64 run to t = 0.2 (0 skips it)")
     ap.add_argument("--igr-arith", default="dw", choices=["both", "dw", "dfma"],
-                    help="engine form(s) of the IGR measurement (the CG itself runs in FP64 "
-                         "fused multiply-adds in both)")
+                    help="engine form(s) of the IGR measurement (dw: the CG's gathers in "
+                         "double-word sums, dfma: in FP64 fused multiply-adds)")
     ap.add_argument("--vortex-side", type=int, default=512,
                     help="nodes per side of the vortex measurement (0 skips it)")
     ap.add_argument("--adj-steps", type=int, default=500,
@@ -743,7 +743,7 @@ def roofline(prof, n, prec, hv, peaks, arith=None, tag=None):
     """Roofline of the kernel with the largest share of the profiled steps: algorithmic
     bytes per launch / its average CUDA-event duration, against the measured HBM copy
     bandwidth; for the FP64 form also its multiply-adds per second against the measured
-    FP64 (DFMA arithmetic) or FP32 (double-word arithmetic, 12 FP32 operations per
+    FP64 (DFMA arithmetic) or FP32 (double-word arithmetic, 10 FP32 operations per
     product) rate."""
     name = max(prof, key=lambda k: prof[k][0])
     ms, launches = prof[name]
@@ -769,12 +769,12 @@ def roofline(prof, n, prec, hv, peaks, arith=None, tag=None):
                                  "frac": g / pk, "fma_per_node": fmas,
                                  "peak_source": "mft_measure_fma_rate (this run)"}
         else:
-            pk = peaks["fma_rates"]["fp32"] / 12.0
+            pk = peaks["fma_rates"]["fp32"] / 10.0
             out["fp32_issue"] = {"achieved_gproducts_s": g / 1e9,
                                  "peak_gproducts_s": pk / 1e9, "frac": g / pk,
                                  "products_per_node": fmas,
-                                 "note": "double-word product + compensated sum = 12 FP32 "
-                                         "operations; peak = measured FP32 FMA rate / 12"}
+                                 "note": "double-word product + compensated sum = 10 FP32 "
+                                         "operations; peak = measured FP32 FMA rate / 10"}
     return out
 
 

@@ -236,9 +236,9 @@ __global__ void __launch_bounds__(kBlock) k_igr_flux(IgrArgs a) {
 // (no pass of its own), and the operator's gather walks the row groups in the opposite order of
 // the direction's, so that the weights one reads last are still in L2 for the other (165 MB of
 // weights at 262,144 nodes against 129 MB of L2).  Each kernel is the programmatic dependent of
-// the one before (what that one wrote is read past L1, after pdl_wait).  One solve of 20
-// iterations at 262,144 nodes: 1947 -> 1219 us (the order of the groups alone: 1604 -> 1511
-// when it was measured).
+// the one before (what that one wrote is read past L1, after pdl_wait).  One solve of
+// 14 iterations (of at most 20) at 262,144 nodes: 1947 -> 1219 us (the order of the groups
+// alone: 1604 -> 1511 when it was measured); where all 20 run, 2.44 -> 1.63 ms per rhs!.
 
 // Per node: rinv and the records of the right-hand side's gather, chunks (v1, v2), (rho, rho).
 __global__ void k_igr_prim_dw(int64_t n, const double* __restrict__ u, float4* rec, double* rinv) {
