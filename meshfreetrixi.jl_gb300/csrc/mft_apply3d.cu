@@ -102,6 +102,7 @@ __global__ void __launch_bounds__(kBlock) k_fwd3_f64(FwdArgs a) {
 // zz, ez).  The state is split on the integer pipe.
 __global__ void k_prep_euler3d_dw(int64_t n, float2 gm1, const double* __restrict__ u,
                                   float4* __restrict__ F) {
+  pdl_trigger();  // the gather may be launched: it waits for this kernel before it reads F
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= n) return;
   const double* ui = u + i * 5;
@@ -156,6 +157,8 @@ static __device__ __forceinline__ void accum3(Sums3& s, float4 wxy, float2 wz, c
 // gathers directly.  Both read the same records in the same order: the same sums.
 // Bound by latency and issue of the packed FP32 products; the row's first weights are requested
 // before the staging, whose wait then covers theirs: 262k nodes 100 us -> 92.5 between events.
+// They are also requested before the flux kernel has ended (pdl_wait stands before the first
+// read of its records, and of anything else that is not constant): rhs! 133.1 -> 129.9 us.
 template <bool HALO>
 __global__ void __launch_bounds__(HALO ? kHaloRows : kBlock, 2) k_fwd3_dw(FwdArgs a) {
   const int64_t r = blockIdx.x * (int64_t)(HALO ? (int)blockDim.x : kBlock) + threadIdx.x;
@@ -180,7 +183,10 @@ __global__ void __launch_bounds__(HALO ? kHaloRows : kBlock, 2) k_fwd3_dw(FwdArg
   if (HALO) {
     if (__ldg(a.ell.halo_off + blockIdx.x + 1) > __ldg(a.ell.halo_off + blockIdx.x))
       pipelined_open<4>(len, ahead, load);
+    pdl_wait();
     staged = stage_halo<kRec3>(a.ell, hsm3, [&](int k, int64_t c) { return F4 + c * kRec3 + k; });
+  } else {
+    pdl_wait();
   }
   if (!live) return;
   const int hs = a.ell.halo_stride;
@@ -230,7 +236,7 @@ void launch_prep_euler3d_dw(int64_t n, double gamma, const double* u, float2* F,
   MFT_LAUNCH_CHECK();
 }
 
-void launch_fwd3_dw(const FwdArgs& a, cudaStream_t s) {
+void launch_fwd3_dw(const FwdArgs& a, cudaStream_t s, bool pdl) {
   if (a.n <= 0) return;
   MFT_REQUIRE(a.V == 5 && a.Fdw && a.wxydw && a.wzdw && a.final_epilogue,
               MFT_ERR_STATE, "double-word 3D gather: arguments not set");
@@ -249,9 +255,9 @@ void launch_fwd3_dw(const FwdArgs& a, cudaStream_t s) {
                                       (int)(kRec3 * kHaloMax * sizeof(float4))));
     }
     const int rows = a.ell.halo_rows;
-    k_fwd3_dw<true><<<grid_for(a.n, rows), rows, smem, s>>>(a);
+    launch_k(k_fwd3_dw<true>, grid_for(a.n, rows), rows, smem, s, pdl, a);
   } else {
-    k_fwd3_dw<false><<<grid_for(a.n, kBlock), kBlock, 0, s>>>(a);
+    launch_k(k_fwd3_dw<false>, grid_for(a.n, kBlock), kBlock, 0, s, pdl, a);
   }
   MFT_LAUNCH_CHECK();
 }

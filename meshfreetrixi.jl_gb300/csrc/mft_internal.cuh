@@ -346,7 +346,8 @@ void launch_fwd3(const FwdArgs& a, cudaStream_t s);
 // chunks) and the gather over the weights a.wxydw, a.wzdw.
 void launch_prep_euler3d_dw(int64_t n, double gamma, const double* u, float2* F,
                             cudaStream_t s);
-void launch_fwd3_dw(const FwdArgs& a, cudaStream_t s);
+// pdl: the launch before in the stream is launch_prep_euler3d_dw (nothing between)
+void launch_fwd3_dw(const FwdArgs& a, cudaStream_t s, bool pdl);
 // Double-word forms (mft_apply_dw.cu): per-node flux and state pairs, forward gather,
 // transpose gather.
 void launch_prep_euler_dw(int64_t n, double gamma, const double* u, float2* F, float2* U,
