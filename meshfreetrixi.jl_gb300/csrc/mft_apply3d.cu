@@ -151,7 +151,7 @@ static __device__ __forceinline__ void accum3(Sums3& s, float4 wxy, float2 wz, c
 
 // du_i = -sum_j (Dx_ij F_x + Dy_ij F_y + Dz_ij F_z)(node j) as compensated sums of
 // double-word products (mft_dw.cuh), the stage epilogue in FP64.  Per stencil entry: three
-// weight pairs and the neighbour's 112-byte flux record.  HALO: one block per row group
+// weight pairs and the neighbour's 112-byte flux record.  One block per row group
 // (ell.halo_rows rows) first stages the group's neighbour records in shared memory (seven
 // 16-byte chunks each, mft_halo.cuh) and reads them from there; a group without a list
 // gathers directly.  Both read the same records in the same order: the same sums.
@@ -159,10 +159,11 @@ static __device__ __forceinline__ void accum3(Sums3& s, float4 wxy, float2 wz, c
 // before the staging, whose wait then covers theirs: 262k nodes 100 us -> 92.5 between events.
 // They are also requested before the flux kernel has ended (pdl_wait stands before the first
 // read of its records, and of anything else that is not constant): rhs! 133.1 -> 129.9 us.
-template <bool HALO>
-__global__ void __launch_bounds__(HALO ? kHaloRows : kBlock, 2) k_fwd3_dw(FwdArgs a) {
-  const int64_t r = blockIdx.x * (int64_t)(HALO ? (int)blockDim.x : kBlock) + threadIdx.x;
-  const float4* __restrict__ F4 = reinterpret_cast<const float4*>(a.Fdw);
+// The records are written while this grid is resident, so no read of them may take the
+// read-only path (__ldg): asynchronous copies or __ldcg.
+__global__ void __launch_bounds__(kHaloRows, 2) k_fwd3_dw(FwdArgs a) {
+  const int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  const float4* F4 = reinterpret_cast<const float4*>(a.Fdw);
   extern __shared__ float4 hsm3[];
   const bool live = r < a.n;
   const int64_t i = live ? ell_node(a.ell, r) : 0;
@@ -179,21 +180,17 @@ __global__ void __launch_bounds__(HALO ? kHaloRows : kBlock, 2) k_fwd3_dw(FwdArg
     e.wxy = __ldg(a.wxydw + base + j * 32);
     e.wz = __ldg(a.wzdw + base + j * 32);
   };
-  bool staged = false;
-  if (HALO) {
-    if (__ldg(a.ell.halo_off + blockIdx.x + 1) > __ldg(a.ell.halo_off + blockIdx.x))
-      pipelined_open<4>(len, ahead, load);
-    pdl_wait();
-    staged = stage_halo<kRec3>(a.ell, hsm3, [&](int k, int64_t c) { return F4 + c * kRec3 + k; });
-  } else {
-    pdl_wait();
-  }
+  if (__ldg(a.ell.halo_off + blockIdx.x + 1) > __ldg(a.ell.halo_off + blockIdx.x))
+    pipelined_open<4>(len, ahead, load);
+  pdl_wait();
+  const bool staged =
+      stage_halo<kRec3>(a.ell, hsm3, [&](int k, int64_t c) { return F4 + c * kRec3 + k; });
   if (!live) return;
   const int hs = a.ell.halo_stride;
   Sums3 f;
   f.f04 = f.f12 = f.f3 = dw::zero2();
   f.f3z = dw::zero();
-  if (HALO && staged) {
+  if (staged) {
     pipelined_run<4>(len, ahead, load, [&](const Streamed& e) {
       float4 q[kRec3];
 #pragma unroll
@@ -210,7 +207,7 @@ __global__ void __launch_bounds__(HALO ? kHaloRows : kBlock, 2) k_fwd3_dw(FwdArg
       const float2 wz = __ldg(a.wzdw + p);
       float4 q[kRec3];
 #pragma unroll
-      for (int k = 0; k < kRec3; ++k) q[k] = __ldg(F4 + c * kRec3 + k);
+      for (int k = 0; k < kRec3; ++k) q[k] = __ldcg(F4 + c * kRec3 + k);
       accum3(f, wxy, wz, q);
     }
   }
@@ -240,25 +237,23 @@ void launch_fwd3_dw(const FwdArgs& a, cudaStream_t s, bool pdl) {
   if (a.n <= 0) return;
   MFT_REQUIRE(a.V == 5 && a.Fdw && a.wxydw && a.wzdw && a.final_epilogue,
               MFT_ERR_STATE, "double-word 3D gather: arguments not set");
-  if (a.ell.halo_off && a.ell.halo_rows > 0) {
-    // one block per row group, seven chunks of the longest list in dynamic shared memory
-    // (above 48 KB a per-kernel opt-in, made once per device)
-    const size_t smem = (size_t)kRec3 * a.ell.halo_stride * sizeof(float4);
-    if (smem > 48 * 1024) {
-      static std::mutex mu;
-      static std::set<int> done;
-      int dev = 0;
-      MFT_CUDA(cudaGetDevice(&dev));
-      std::lock_guard<std::mutex> lock(mu);
-      if (done.insert(dev).second)
-        MFT_CUDA(cudaFuncSetAttribute(k_fwd3_dw<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)(kRec3 * kHaloMax * sizeof(float4))));
-    }
-    const int rows = a.ell.halo_rows;
-    launch_k(k_fwd3_dw<true>, grid_for(a.n, rows), rows, smem, s, pdl, a);
-  } else {
-    launch_k(k_fwd3_dw<false>, grid_for(a.n, kBlock), kBlock, 0, s, pdl, a);
+  MFT_REQUIRE(a.ell.halo_off && a.ell.halo_rows > 0, MFT_ERR_STATE,
+              "double-word 3D gather: row groups not built");
+  // one block per row group, seven chunks of the longest list in dynamic shared memory
+  // (above 48 KB a per-kernel opt-in, made once per device)
+  const size_t smem = (size_t)kRec3 * a.ell.halo_stride * sizeof(float4);
+  if (smem > 48 * 1024) {
+    static std::mutex mu;
+    static std::set<int> done;
+    int dev = 0;
+    MFT_CUDA(cudaGetDevice(&dev));
+    std::lock_guard<std::mutex> lock(mu);
+    if (done.insert(dev).second)
+      MFT_CUDA(cudaFuncSetAttribute(k_fwd3_dw, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)(kRec3 * kHaloMax * sizeof(float4))));
   }
+  const int rows = a.ell.halo_rows;
+  launch_k(k_fwd3_dw, grid_for(a.n, rows), rows, smem, s, pdl, a);
   MFT_LAUNCH_CHECK();
 }
 
