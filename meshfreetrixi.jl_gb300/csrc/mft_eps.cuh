@@ -73,7 +73,9 @@ static __device__ __forceinline__ double eps_value(const EpsArgs& a, int64_t i,
                                                    const double* dpv_in) {
   const int sg = a.seg_id ? a.seg_id[i] : 0;
   const double h = a.seg_h ? a.seg_h[sg] : a.h;
-  const double* __restrict__ norms = a.norms + (a.seg_id ? sg * 2 * V : 0);
+  // not __restrict__: the reductions may still write them while the gather that waits for them
+  // is resident, so no read may take the read-only path
+  const double* norms = a.norms + (a.seg_id ? sg * 2 * V : 0);
   const int si = a.tab ? a.tab[*a.ctr].si_eps : a.success_iter;
   const bool rv = a.kind == MFT_SRC_RV && si != 0;
   double eps_rv = 0.0;
