@@ -136,18 +136,20 @@ static __device__ __forceinline__ double eps_value(const EpsArgs& a, int64_t i,
   // The final comparison is on bit patterns of values >= 0 (or NaN, which fails it).
   // The same test in FP32 first (the FP64 pipe is the scarce one): its terms carry less than
   // 1e-5 of relative error (mm <= E rho is asked with that margin too, so the difference keeps
-  // half of E rho), so lhs < (1 - 1e-4) rhs in FP32 proves the FP64 inequality; the ranges keep
-  // the FP32 terms normal (lhs may underflow: it is then below rhs).
+  // half of E rho), so lhs < (1 - 1e-4) rhs in FP32 proves the FP64 inequality.  The ranges keep
+  // every FP32 factor normal: uwc from 1e-15 (its square from 1e-30), rho from 1e-6, w from 1e-18
+  // (what underflowed inside w is far below that).  eps_rv may round in the subnormal range, by
+  // less than the smallest normal float, which is added; lhs may underflow: it is then below rhs.
   bool done = false;
   if (V == 4 && rv_finite) {
     const float rf = fpconv::d2f(rho), ef = fpconv::d2f(en);
     const float f1 = fpconv::d2f(m1), f2 = fpconv::d2f(m2), uf = fpconv::d2f(uwc);
-    const float er = fpconv::d2f(eps_rv) * rf;
+    const float er = (fpconv::d2f(eps_rv) + 1.17549435e-38f) * rf;
     const float mm = f1 * f1 + f2 * f2, erho = ef * rf;
     float w = mm;
     if (mm <= 0.99999f * erho) w = mm + a.gg1_32 * (erho - 0.5f * mm);
     const float rhs = uf * uf * w;
-    if (rf >= 1e-6f && uf > 0.0f && ef == ef && w >= 1e-18f && rhs >= 1e-30f && rhs <= 1e30f &&
+    if (rf >= 1e-6f && uf >= 1e-15f && ef == ef && w >= 1e-18f && rhs >= 1e-30f && rhs <= 1e30f &&
         er * er < 0.9999f * rhs)
       return eps_rv;
   }
