@@ -177,8 +177,8 @@ static __device__ __forceinline__ void lam_chunks(const double* __restrict__ lam
   out[1] = dw::chunk(dw::split(l[2]), dw::split(l[3]));
 }
 
-// M2 lam as double-word chunks (two per node): the cotangent the direct double-word adjoint
-// gather reads, masked once per node instead of once per stencil entry.
+// M2 lam as double-word chunks (two per node): the cotangent that rows outside the staged groups
+// read, masked and split once per node instead of once per stencil entry.
 template <bool BC>
 __global__ void k_lam_pairs(int64_t n, const double* __restrict__ lam, BcDev bc,
                             float4* __restrict__ out) {
@@ -191,9 +191,11 @@ __global__ void k_lam_pairs(int64_t n, const double* __restrict__ lam, BcDev bc,
 // gathers; the sums over the reverse adjacency in pairs, the node part in FP64).  HV 0
 // (no hyperviscosity) or 2 (Flyer, whose term gathers the same M2 lam).
 // HALO: blocks of one row group form the group's neighbour cotangents while staging them in
-// shared memory (a group without a list forms them per entry); same sums, same order.  A group's
-// neighbours are 1.8 times its rows, the splits run on the integer pipe, and the kernel that
-// wrote them for every node before is gone (one launch per stage, 65,536 nodes).  With the
+// shared memory; same sums, same order.  A group's neighbours are 1.8 times its rows, the splits
+// run on the integer pipe, and where every group is staged the kernel that writes them for every
+// node (k_lam_pairs) is not launched (one launch per stage, 65,536 nodes).  A group without a list
+// reads that kernel's chunks, one 32-byte load per entry: forming them per entry took 169 us
+// against 140 at 262,144 scattered nodes, none staged.  With the
 // streamed loads in groups of kAdjGroup ahead the gather and that kernel took 26.4 us between
 // events against 29.2 (groups of 2 / 3 / 4 / 5: 27.4 / 27.0 / 26.3 / 27.2); without that kernel and
 // with the first entries requested before the staging 23.9.
@@ -201,7 +203,7 @@ constexpr int kAdjGroup = 6;
 template <bool BC, int HV, bool HALO>
 __global__ void __launch_bounds__(HALO ? kHaloRows : kBlock) k_adj_dw(AdjArgs a) {
   const int64_t row = blockIdx.x * (int64_t)(HALO ? (int)blockDim.x : kBlock) + threadIdx.x;
-  const float4* __restrict__ L4 = reinterpret_cast<const float4*>(a.lamdw);
+  const float* __restrict__ L = reinterpret_cast<const float*>(a.lamdw);
   extern __shared__ float4 hsm[];
   const bool live = row < a.n;
   const int64_t i = live ? ell_node(a.ell, row) : 0;
@@ -258,14 +260,8 @@ __global__ void __launch_bounds__(HALO ? kHaloRows : kBlock) k_adj_dw(AdjArgs a)
     });
   else
     pipelined_row<2, Streamed>(len, load, [&](const Streamed& e) {
-      float4 l[2];
-      if (HALO) {
-        lam_chunks<BC>(a.lam, a.bc, e.at, l);
-      } else {
-        l[0] = __ldg(L4 + (int64_t)e.at * 2);
-        l[1] = __ldg(L4 + (int64_t)e.at * 2 + 1);
-      }
-      take(e, l[0], l[1]);
+      const F8 l = ldg_f8(L + (int64_t)e.at * 8);
+      take(e, l.lo, l.hi);
     });
   // the Jacobian product in double-word arithmetic from the sums as pairs
   float2 gxp[4], gyp[4];
@@ -347,7 +343,9 @@ void launch_adj_dw(const AdjArgs& a, float2* lam_pairs, bool staged, cudaStream_
   if (a.n <= 0) return;
   MFT_REQUIRE(a.V == 4 && a.eq == MFT_EQ_EULER2D && a.hv != 1, MFT_ERR_UNSUPPORTED,
               "double-word adjoint gather: 2D Euler without Tominec hyperviscosity");
-  if (!(staged && a.ell.halo_off)) {
+  MFT_REQUIRE(lam_pairs || (staged && a.ell.halo_off), MFT_ERR_STATE,
+              "direct adjoint gather: no scratch for the cotangent's pairs");
+  if (lam_pairs) {
     const unsigned gn = grid_for(a.n, 256);
     if (a.has_bc) k_lam_pairs<true><<<gn, 256, 0, s>>>(a.n, a.lam, a.bc, reinterpret_cast<float4*>(lam_pairs));
     else k_lam_pairs<false><<<gn, 256, 0, s>>>(a.n, a.lam, a.bc, reinterpret_cast<float4*>(lam_pairs));

@@ -2778,9 +2778,11 @@ void eval_rhs_adjoint(mft_ctx* c, const double* u, const double* lam, int kind, 
     ensure_device_ops(c);
     a.wxydw = reinterpret_cast<const float4*>(c->rwdw[0].p);
     a.whdw = hv == 2 ? c->rwdw[kSlotHv].p : nullptr;
-    c->adj_lamdw.alloc((size_t)c->n * 4);
-    // staged unless a fixed direct variant of the double-word gathers is requested
+    // staged unless a fixed direct variant of the double-word gathers is requested; the
+    // cotangent's pairs are written only where some row group reads them
     const bool staged = !(c->dw_variant >= 0 && c->dw_variant < 6);
+    if (staged && c->rev.halo_staged == c->rev.halo_groups) c->adj_lamdw.release();
+    else c->adj_lamdw.alloc((size_t)c->n * 4);
     a.ell = c->rev.view();
     launch_adj_dw(a, c->adj_lamdw.p, staged, s);
   } else {

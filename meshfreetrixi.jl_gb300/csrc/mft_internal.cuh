@@ -469,8 +469,9 @@ struct AdjArgs {
   const float2* lamdw;  // M2 lam as pairs (set by launch_adj_dw)
 };
 void launch_adj_f64(const AdjArgs& a, cudaStream_t s);
-// The same product with the sums in double-word arithmetic; lam_pairs: n x 4 pair scratch;
-// staged: each row group's neighbour pairs staged in shared memory (when halos exist).
+// The same product with the sums in double-word arithmetic; staged: each row group's neighbour
+// pairs staged in shared memory (when halos exist); lam_pairs: n x 4 pair scratch, or null where
+// every row is staged.
 void launch_adj_dw(const AdjArgs& a, float2* lam_pairs, bool staged, cudaStream_t s);
 // q_i = sum_j lap[i,j] (M2 lam)_j over the forward layout (Tominec adjoint).
 void launch_lap_masked(int64_t n, EllView fwd, const double* wl, const double* lam, int V,
