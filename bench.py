@@ -101,8 +101,8 @@ def parse():
     ap.add_argument("--riemann-side", type=int, default=1024,
                     help="nodes per side of the Riemann FP32/FP64 run to t = 0.2 (0 skips it)")
     ap.add_argument("--igr-arith", default="dw", choices=["both", "dw", "dfma"],
-                    help="engine form(s) of the IGR measurement (dw: the CG's gathers in "
-                         "double-word sums, dfma: in FP64 fused multiply-adds)")
+                    help="engine form(s) of the IGR measurement (the CG itself runs in FP64 "
+                         "fused multiply-adds in both)")
     ap.add_argument("--vortex-side", type=int, default=512,
                     help="nodes per side of the vortex measurement (0 skips it)")
     ap.add_argument("--adj-steps", type=int, default=500,

@@ -945,20 +945,24 @@ static void check_kernel_errors(mft_ctx* c, bool brought = false) {
   }
 }
 
-// Work buffers of the IGR source.
-static void ensure_igr(mft_ctx* c) {
+// Work buffers of the IGR source; returns the staged update's largest grid (two blocks of 256
+// threads per SM leave its last-block sum short).
+static unsigned ensure_igr(mft_ctx* c) {
   const size_t n = (size_t)c->n;
-  c->igr_prim.alloc(n * 4);
+  int nsm = 0;
+  MFT_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device));
+  c->igr_prim.alloc(n * 3);
   for (auto* b : {&c->igr_rinv, &c->igr_x, &c->igr_r, &c->igr_u0, &c->igr_u1, &c->igr_c})
     b->alloc(n);
   c->igr_t.alloc(n * 2);
   c->igr_add.alloc(n * 2);
-  c->igr_partial.alloc((n + kBlockHost - 1) / kBlockHost + 512);
+  c->igr_partial.alloc((n + kBlockHost - 1) / kBlockHost + 2 * nsm);
   if (!c->igr_counter.p) {
     c->igr_counter.alloc(1);
     c->igr_counter.zero(c->stream);
   }
   c->igr_sc.alloc(1);
+  return 2u * (unsigned)nsm;
 }
 
 void eval_rhs(mft_ctx* c, double* us, float* us32, double t, const Epilogue& ep_in) {
@@ -1119,13 +1123,15 @@ void eval_rhs(mft_ctx* c, double* us, float* us32, double t, const Epilogue& ep_
   if (ig >= 0) {
     MFT_REQUIRE(c->eq == MFT_EQ_EULER2D && c->dim == 2, MFT_ERR_UNSUPPORTED,
                 "the IGR source needs the 2D Euler equations");
-    ensure_igr(c);
     IgrArgs ia{};
+    ia.update_blocks = ensure_igr(c);
+    // the staged kernels in the double-word engine form where every row group is staged: a group
+    // without a list would form the direction at every entry
+    ia.staged = dw && c->fwd.halo_groups > 0 && c->fwd.halo_staged == c->fwd.halo_groups;
     ia.n = n;
     ia.ell = c->fwd.view();
     ia.wx = c->fw[0].p;
     ia.wy = c->fw[1].p;
-    ia.wxydw = dw ? reinterpret_cast<const float4*>(c->fwdw[0].p) : nullptr;
     ia.alpha = c->src_par[ig * 4];
     ia.maxiter = (int)c->src_par[ig * 4 + 1];
     ia.prim = c->igr_prim.p;

@@ -7,15 +7,14 @@
 //       conjugate gradients from sigma = 0, at most maxiter iterations, relative
 //       tolerance sqrt(eps) (the in-place cg! the reference intends at :189);
 //   du[rho v1] -= Dx sigma, du[rho v2] -= Dy sigma (:214-237).
-// The CG runs as a fixed sequence of kernels (four per iteration) whose scalars live in
-// device memory; once converged, the remaining kernels return at entry, so one rhs!
-// evaluation is a fixed launch sequence that a CUDA graph can hold.  Reductions are
-// block partials finished by the last block in a fixed order (deterministic).
+// The CG runs as a fixed sequence of kernels (four per iteration, or three where every row group
+// is staged) whose scalars live in device memory; once converged, the remaining kernels return
+// at entry, so one rhs! evaluation is a fixed launch sequence that a CUDA graph can hold.
+// Reductions are block partials added in a fixed order (deterministic).
 #include <algorithm>
 #include <cfloat>
 
 #include "mft_device.cuh"
-#include "mft_dw.cuh"
 #include "mft_halo.cuh"
 
 namespace mft {
@@ -225,32 +224,23 @@ __global__ void __launch_bounds__(kBlock) k_igr_flux(IgrArgs a) {
   a.add[i * 2 + 1] = -sy;
 }
 
-// ---------------------------------------------------------------- double-word form
+// ---------------------------------------------------------------- staged form
 //
-// The same iteration with the gathers' sums in double-word arithmetic over the staged layout
-// (mft_dw.cuh, mft_halo.cuh), where the engine's FP64 form uses it; the CG scalars, vectors and
-// their updates stay FP64.  The FP64 gathers issued 70 multiply-adds per node on a pipe that
-// takes 35 us for 262,144 nodes of them and fetched every neighbour value from L2; here one
-// packed product serves an entry and the gathers are bound by the 630 B of weights and
-// positions per node.  What the iteration spends: the new direction is formed while staging
-// (no pass of its own), and the operator's gather walks the row groups in the opposite order of
-// the direction's, so that the weights one reads last are still in L2 for the other (165 MB of
-// weights at 262,144 nodes against 129 MB of L2).  Each kernel is the programmatic dependent of
-// the one before (what that one wrote is read past L1, after pdl_wait).  One solve of
-// 14 iterations (of at most 20) at 262,144 nodes: 1947 -> 1219 us (the order of the groups
-// alone: 1604 -> 1511 when it was measured); where all 20 run, 2.44 -> 1.63 ms per rhs!.
-
-// Per node: rinv and the records of the right-hand side's gather, chunks (v1, v2), (rho, rho).
-__global__ void k_igr_prim_dw(int64_t n, const double* __restrict__ u, float4* rec, double* rinv) {
-  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const double2 a = reinterpret_cast<const double2*>(u)[i * 2];
-  const double m2 = u[i * 4 + 2];
-  const float2 rho = dw::split(a.x), r = dw::recip(rho);
-  rec[i * 2] = dw::chunk(dw::mul(dw::split(a.y), r), dw::mul(dw::split(m2), r));
-  rec[i * 2 + 1] = dw::chunk(rho, rho);
-  rinv[i] = ddiv(1.0, a.x);
-}
+// The same iteration in three kernels over the staged layout (mft_halo.cuh), for clouds whose
+// row groups are all staged; the arithmetic is the kernels' above, operation by operation, but
+// for the order in which the blocks' parts of the two dot products are added.  (In double-word
+// sums, as the engine's own gathers, the solve was faster still, 1.43 ms for the case below, but
+// its part of du was 50 to 100 times further from a quad-precision solve, up to 1.4e-10 of its
+// largest value against 2e-12, and at alpha = 20 h^2 du as a whole up to eight times.)
+// What bounds it: the FP64 pipe, 37 us for the 70 multiply-adds per node of one gather at 262,144
+// nodes, and the 630 B of weights and positions per node.  The new direction is formed while
+// staging (no pass of its own), the gathers read neighbours from shared memory, and the
+// operator's gather walks the row groups in the opposite order of the direction's, so that the
+// weights one reads last are still in L2 for the other (165 MB of weights at 262,144 nodes
+// against 129 MB of L2).  Each kernel is the programmatic dependent of the one before: what that
+// one wrote (vectors and CG scalars) is read after pdl_wait and past L1.  One rhs! with a solve
+// of 16 iterations (of at most 20) at 262,144 nodes: 2.25 ms with the kernels above, 1.90 with
+// these; of 20: 2.67 / 2.25, and at 16,384 nodes 0.87 / 0.46, at 65,536 1.05 / 1.00.
 
 // Sum of x over the block, in thread 0 (fixed order).
 __device__ __forceinline__ double block_total(double x) {
@@ -288,169 +278,114 @@ __device__ bool last_block_sum(double x, double* partial, unsigned* counter, dou
 }
 
 // Entries per register group of the gathers, and blocks per SM their registers are capped for.
-// Measured (262,144 nodes, one solve): groups of 2 / 3 / 4 / 5 uncapped 1371 / 1322 / 1398 / 1450
-// us; 3 capped at four blocks 1219, 2 at five 1507 (spills), 5 at three 1369.
-constexpr int kIgrGroup = 3, kIgrBlocks = 4;
-
-// One entry of a row's stream.
-struct IgrStream {
-  int lc;
-  float4 wxy;
-};
+// One rhs! of 20 iterations at 16,384 / 65,536 / 262,144 nodes, us: 3 entries at four blocks 571 /
+// 1304 / 2300, 4 at three 586 / 1168 / 2344, 5 at three 466 / 998 / 2250, 6 at three 481 / 1035 /
+// 2409, 6 at two 614 / 995 / 2544, 3 at five 575 / 1423 / 2224.
+constexpr int kIgrGroup = 5, kIgrBlocks = 3;
 
 // The gather of row group `group` (the block's): per entry of this thread's row
-// sum(weights, record of the neighbour), the record staged in shared memory as chunk(c) or, in a
-// group without a list, chunk(c) itself.  What does not depend on the kernel before -- the row,
-// the list, and the first 2 G entries' weights -- is requested before wait(), which returns
-// whether there is anything to do: the weights' latency and the launch then overlap that
-// kernel's tail and the staging.  (STAGED: two loops, because one that chose the source per entry loaded
-// through generic addresses.)  Every thread of the block must call it.
-template <int G, bool STAGED, typename Wait, typename Chunk, typename Sum>
-__device__ __forceinline__ bool igr_gather_as(const IgrArgs& a, int64_t r, int h0, int nh, float4* sm,
-                                              Wait wait, Chunk chunk, Sum sum) {
+// sum(w_x, w_y, value of the neighbour), the values staged in shared memory as value(c).  What
+// does not depend on the kernel before -- the row, the list, and the first 2 G entries' weights
+// -- is requested before wait(), which returns whether there is anything to do: the weights'
+// latency and the launch then overlap that kernel's tail and the staging.  Every thread of the
+// block must call it.
+struct IgrStream {
+  int lc;
+  double wx, wy;
+};
+template <typename T, typename Wait, typename Value, typename Sum>
+__device__ __forceinline__ bool igr_gather(const IgrArgs& a, unsigned group, T* sm, Wait wait,
+                                           Value value, Sum sum) {
+  const int h0 = __ldg(a.ell.halo_off + group), nh = __ldg(a.ell.halo_off + group + 1) - h0;
+  const int64_t r = group * (int64_t)blockDim.x + threadIdx.x;  // layout row
   const bool live = r < a.n;
   const int64_t base = live ? a.ell.slice_off[r >> 5] + (r & 31) : 0;
   const int len = live ? a.ell.row_len[r] : 0;
-  IgrStream e[2][G];
+  IgrStream e[2][kIgrGroup];
   auto load = [&](IgrStream& x, int j) {
     const int64_t p = base + (int64_t)j * 32;
-    x.lc = STAGED ? (int)__ldg(a.ell.lcol + p) : __ldg(a.ell.col + p);
-    x.wxy = __ldg(a.wxydw + p);
+    x.lc = __ldg(a.ell.lcol + p);
+    x.wx = __ldg(a.wx + p);
+    x.wy = __ldg(a.wy + p);
   };
-  auto use = [&](const IgrStream& x) { sum(x.wxy, STAGED ? sm[x.lc] : chunk((int64_t)x.lc)); };
   const int q0 = threadIdx.x, q1 = q0 + blockDim.x;
-  const int c0 = STAGED && q0 < nh ? __ldg(a.ell.halo_col + h0 + q0) : -1;
-  const int c1 = STAGED && q1 < nh ? __ldg(a.ell.halo_col + h0 + q1) : -1;
-  pipelined_open<G>(len, e, load);
+  const int c0 = q0 < nh ? __ldg(a.ell.halo_col + h0 + q0) : -1;
+  const int c1 = q1 < nh ? __ldg(a.ell.halo_col + h0 + q1) : -1;
+  pipelined_open<kIgrGroup>(len, e, load);
   if (!wait()) return false;
-  if (STAGED) {
-    const float4 v0 = c0 >= 0 ? chunk(c0) : make_float4(0.f, 0.f, 0.f, 0.f);
-    const float4 v1 = c1 >= 0 ? chunk(c1) : make_float4(0.f, 0.f, 0.f, 0.f);
-    if (c0 >= 0) sm[q0] = v0;
-    if (c1 >= 0) sm[q1] = v1;
-    for (int q = q1 + blockDim.x; q < nh; q += blockDim.x)
-      sm[q] = chunk((int64_t)__ldg(a.ell.halo_col + h0 + q));
-    __syncthreads();
-  }
-  pipelined_run<G>(len, e, load, use);
+  const T v0 = c0 >= 0 ? value(c0) : T{};
+  const T v1 = c1 >= 0 ? value(c1) : T{};
+  if (c0 >= 0) sm[q0] = v0;
+  if (c1 >= 0) sm[q1] = v1;
+  for (int q = q1 + blockDim.x; q < nh; q += blockDim.x)
+    sm[q] = value((int64_t)__ldg(a.ell.halo_col + h0 + q));
+  __syncthreads();
+  pipelined_run<kIgrGroup>(len, e, load,
+                           [&](const IgrStream& x) { sum(x.wx, x.wy, sm[x.lc]); });
   return true;
 }
-template <int G, typename Wait, typename Chunk, typename Sum>
-__device__ __forceinline__ bool igr_gather(const IgrArgs& a, unsigned group, float4* sm, Wait wait,
-                                           Chunk chunk, Sum sum) {
-  const int h0 = __ldg(a.ell.halo_off + group), nh = __ldg(a.ell.halo_off + group + 1) - h0;
-  const int64_t r = group * (int64_t)blockDim.x + threadIdx.x;  // layout row
-  if (nh > 0) return igr_gather_as<G, true>(a, r, h0, nh, sm, wait, chunk, sum);
-  return igr_gather_as<G, false>(a, r, h0, nh, sm, wait, chunk, sum);
-}
 
-__global__ void __launch_bounds__(kHaloRows) k_igr_rhs_dw(IgrArgs a) {
-  extern __shared__ float4 sm[];
-  const float4* rec = reinterpret_cast<const float4*>(a.prim);
-  const bool staged = stage_halo<2>(a.ell, sm, [&](int k, int64_t c) { return rec + c * 2 + k; });
-  const int hs = a.ell.halo_stride;
-  const int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;  // layout row
-  double rr = 0.0;
-  if (r < a.n) {
-    const int64_t i = ell_node(a.ell, r);
-    const int64_t base = a.ell.slice_off[r >> 5] + (r & 31);
-    dw::Acc2 sx = dw::zero2(), sy = dw::zero2();  // (Dx v1, Dx v2), (Dy v1, Dy v2)
-    dw::Acc sr = dw::zero();
-    auto sum = [&](float4 wxy, float4 v, float4 d) {
-      const float2 wx = dw::chunk_a(wxy);
-      dw::fma_acc2(sx, dw::both(wx), dw::pair2(v));
-      dw::fma_acc2(sy, dw::both(dw::chunk_b(wxy)), dw::pair2(v));
-      dw::fma_acc(sr, wx, dw::chunk_a(d));
-    };
-    if (staged) {
-      pipelined_row<3, IgrStream>(
-          a.ell.row_len[r],
-          [&](IgrStream& e, int j) {
-            e.lc = __ldg(a.ell.lcol + base + j * 32);
-            e.wxy = __ldg(a.wxydw + base + j * 32);
-          },
-          [&](const IgrStream& e) {
-            sum(e.wxy, sm[halo_at<2>(0, e.lc, hs)], sm[halo_at<2>(1, e.lc, hs)]);
-          });
-    } else {
-      for (int j = 0; j < a.ell.row_len[r]; ++j) {
-        const int64_t c = __ldg(a.ell.col + base + j * 32);
-        sum(__ldg(a.wxydw + base + j * 32), __ldg(rec + c * 2), __ldg(rec + c * 2 + 1));
-      }
-    }
-    const double dxv1 = dw::to_double(dw::first(sx)), dxv2 = dw::to_double(dw::second(sx));
-    const double dyv1 = dw::to_double(dw::first(sy)), dyv2 = dw::to_double(dw::second(sy));
-    const double tr = dadd(dw::to_double(sr), dyv1);
-    const double tsq = dadd(dadd(dmul(dxv1, dxv1), dmul(dmul(2.0, dyv1), dxv2)), dmul(dyv2, dyv2));
-    const double b = dmul(a.alpha, dadd(dmul(tr, tr), tsq));
-    a.x[i] = 0.0;
-    a.r[i] = b;
-    a.u0[i] = 0.0;
-    rr = dmul(b, b);
-  }
-  double total;
-  if (last_block_sum(rr, a.partial, a.counter, &total)) igr_start(a, total);
-}
-
-// t = rinv (Dx u_new, Dy u_new) as chunks (t1, t2), u_new = r + beta u_old formed while staging
-// and written for the node's own row; or, FLUX, add = -(Dx sigma, Dy sigma).
+// t = rinv (Dx u_new, Dy u_new), u_new = r + beta u_old formed while staging and written for the
+// node's own row; or, FLUX, add = -(Dx sigma, Dy sigma).
 template <bool FLUX>
-__global__ void __launch_bounds__(kHaloRows, kIgrBlocks) k_igr_dir_dw(IgrArgs a, const double* uo, double* un) {
-  extern __shared__ float4 sm[];
+__global__ void __launch_bounds__(kHaloRows, kIgrBlocks) k_igr_dir_staged(IgrArgs a, const double* uo, double* un) {
+  extern __shared__ double2 sm2[];
   pdl_trigger();
   const int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;  // layout row
   const int64_t i = r < a.n ? ell_node(a.ell, r) : 0;
   const double ri = !FLUX && r < a.n ? a.rinv[i] : 0.0;
   double beta = 0.0;
   auto value = [&](int64_t c) { return FLUX ? __ldcg(a.x + c) : dadd(__ldcg(a.r + c), dmul(beta, __ldcg(uo + c))); };
-  dw::Acc2 s = dw::zero2();
-  const bool ran = igr_gather<kIgrGroup>(
-      a, blockIdx.x, sm,
+  double sx = 0.0, sy = 0.0;
+  const bool ran = igr_gather(
+      a, blockIdx.x, reinterpret_cast<double*>(sm2),
       [&] {
         pdl_wait();
-        beta = FLUX ? 0.0 : a.sc->beta;
-        return FLUX || !a.sc->done;
+        beta = FLUX ? 0.0 : __ldcg(&a.sc->beta);
+        return FLUX || !__ldcg(&a.sc->done);
       },
-      [&](int64_t c) {
-        const float2 v = dw::split(value(c));
-        return dw::chunk(v, v);
-      },
-      [&](float4 wxy, float4 v) { dw::fma_acc2(s, dw::pair2(wxy), dw::pair2(v)); });
+      value,
+      [&](double wx, double wy, double v) {
+        sx = fma(wx, v, sx);
+        sy = fma(wy, v, sy);
+      });
   if (!ran || r >= a.n) return;
-  const double sx = dw::to_double(dw::first(s)), sy = dw::to_double(dw::second(s));
   if (FLUX) {
     reinterpret_cast<double2*>(a.add)[i] = make_double2(-sx, -sy);
     return;
   }
   un[i] = value(i);
-  reinterpret_cast<float4*>(a.t)[i] = dw::chunk(dw::split(dmul(ri, sx)), dw::split(dmul(ri, sy)));
+  reinterpret_cast<double2*>(a.t)[i] = make_double2(dmul(ri, sx), dmul(ri, sy));
 }
 
 // c = rinv u_new - alpha (Dx t1 + Dy t2) and the block's part of u_new . c.  Block b takes the
 // group gridDim.x - 1 - b.  The update's blocks add the parts up, each for itself: a last block
 // that did it here would hold every one of the 1024 blocks at a fence and an atomic.
-__global__ void __launch_bounds__(kHaloRows, kIgrBlocks) k_igr_op_dw(IgrArgs a, const double* un) {
-  extern __shared__ float4 sm[];
+__global__ void __launch_bounds__(kHaloRows, kIgrBlocks) k_igr_op_staged(IgrArgs a, const double* un) {
+  extern __shared__ double2 sm2[];
   pdl_trigger();
   const unsigned group = gridDim.x - 1 - blockIdx.x;
-  const float4* t4 = reinterpret_cast<const float4*>(a.t);
+  const double2* t2 = reinterpret_cast<const double2*>(a.t);
   const int64_t r = group * (int64_t)blockDim.x + threadIdx.x;  // layout row
   const int64_t i = r < a.n ? ell_node(a.ell, r) : 0;
   const double ri = r < a.n ? a.rinv[i] : 0.0;
-  dw::Acc2 s = dw::zero2();
-  const bool ran = igr_gather<kIgrGroup>(
-      a, group, sm,
+  double sx = 0.0, sy = 0.0;
+  const bool ran = igr_gather(
+      a, group, sm2,
       [&] {
         pdl_wait();
-        return !a.sc->done;
+        return !__ldcg(&a.sc->done);
       },
-      [&](int64_t c) { return __ldcg(t4 + c); },
-      [&](float4 wxy, float4 v) { dw::fma_acc2(s, dw::pair2(wxy), dw::pair2(v)); });
+      [&](int64_t c) { return __ldcg(t2 + c); },
+      [&](double wx, double wy, double2 t) {
+        sx = fma(wx, t.x, sx);
+        sy = fma(wy, t.y, sy);
+      });
   if (!ran) return;
   double uc = 0.0;
   if (r < a.n) {
     const double ui = __ldcg(un + i);
-    const double ci = dsub(dmul(ri, ui), dmul(a.alpha, dw::sum_double(dw::first(s), dw::second(s))));
+    const double ci = dsub(dmul(ri, ui), dmul(a.alpha, dadd(sx, sy)));
     a.c[i] = ci;
     uc = dmul(ui, ci);
   }
@@ -460,23 +395,26 @@ __global__ void __launch_bounds__(kHaloRows, kIgrBlocks) k_igr_op_dw(IgrArgs a, 
 
 // alpha_cg = res^2 / (u_new . c) from the nparts parts; x += alpha_cg u_new; r -= alpha_cg c;
 // new residual, beta, convergence
-__global__ void __launch_bounds__(kHaloRows) k_igr_update_dw(IgrArgs a, const double* un,
-                                                             unsigned nparts, double* partial) {
+__global__ void __launch_bounds__(kHaloRows) k_igr_update_staged(IgrArgs a, const double* un,
+                                                                 unsigned nparts, double* partial) {
   pdl_trigger();
   pdl_wait();
-  if (a.sc->done) return;
+  if (__ldcg(&a.sc->done)) return;
   __shared__ double al_s;
   double uc = 0.0;
   for (unsigned b = threadIdx.x; b < nparts; b += blockDim.x) uc = dadd(uc, __ldcg(a.partial + b));
   uc = block_total(uc);
-  if (threadIdx.x == 0) al_s = ddiv(dmul(a.sc->res, a.sc->res), uc);
+  if (threadIdx.x == 0) {
+    const double res = __ldcg(&a.sc->res);
+    al_s = ddiv(dmul(res, res), uc);
+  }
   __syncthreads();
   const double al = al_s;
   double rr = 0.0;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < a.n;
        i += (int64_t)gridDim.x * blockDim.x) {
-    a.x[i] = dadd(a.x[i], dmul(al, __ldcg(un + i)));
-    const double r = dsub(a.r[i], dmul(al, __ldcg(a.c + i)));
+    a.x[i] = dadd(__ldcg(a.x + i), dmul(al, __ldcg(un + i)));
+    const double r = dsub(__ldcg(a.r + i), dmul(al, __ldcg(a.c + i)));
     a.r[i] = r;
     rr = dadd(rr, dmul(r, r));
   }
@@ -484,36 +422,31 @@ __global__ void __launch_bounds__(kHaloRows) k_igr_update_dw(IgrArgs a, const do
   if (last_block_sum(rr, partial, a.counter, &total)) igr_next(a, total);
 }
 
-void launch_igr_dw(const IgrArgs& a, const double* u, cudaStream_t s) {
+void launch_igr_staged(const IgrArgs& a, cudaStream_t s) {
   const int rows = a.ell.halo_rows;
   const unsigned g = (unsigned)((a.n + rows - 1) / rows);
-  const size_t one = (size_t)a.ell.halo_stride * sizeof(float4);
-  // the update's grid: two blocks of 256 threads per SM leave its last-block sum short
-  const unsigned gu = std::min<unsigned>((unsigned)((a.n + kHaloRows - 1) / kHaloRows), 304u);
-  k_igr_prim_dw<<<(unsigned)((a.n + 255) / 256), 256, 0, s>>>(a.n, u, reinterpret_cast<float4*>(a.prim), a.rinv);
-  MFT_LAUNCH_CHECK();
-  k_igr_rhs_dw<<<g, rows, 2 * one, s>>>(a);
-  MFT_LAUNCH_CHECK();
+  const size_t one = (size_t)a.ell.halo_stride * sizeof(double);
+  const unsigned gu = std::min<unsigned>((unsigned)((a.n + kHaloRows - 1) / kHaloRows), a.update_blocks);
   for (int it = 0; it < a.maxiter; ++it) {
     const double* uo = (it & 1) ? a.u1 : a.u0;
     double* un = (it & 1) ? a.u0 : a.u1;
-    launch_k(k_igr_dir_dw<false>, g, rows, one, s, true, a, uo, un);
-    launch_k(k_igr_op_dw, g, rows, one, s, true, a, (const double*)un);
-    launch_k(k_igr_update_dw, gu, kHaloRows, 0, s, true, a, (const double*)un, g, a.partial + g);
+    launch_k(k_igr_dir_staged<false>, g, rows, one, s, true, a, uo, un);
+    launch_k(k_igr_op_staged, g, rows, 2 * one, s, true, a, (const double*)un);
+    launch_k(k_igr_update_staged, gu, kHaloRows, 0, s, true, a, (const double*)un, g, a.partial + g);
   }
-  launch_k(k_igr_dir_dw<true>, g, rows, one, s, true, a, (const double*)nullptr, (double*)nullptr);
+  launch_k(k_igr_dir_staged<true>, g, rows, one, s, true, a, (const double*)nullptr, (double*)nullptr);
 }
 
 }  // namespace
 
 void launch_igr(const IgrArgs& a, const double* u, cudaStream_t s) {
   if (a.n <= 0) return;
-  if (a.wxydw && a.ell.halo_off && a.ell.halo_rows > 0) return launch_igr_dw(a, u, s);
   const unsigned g = (unsigned)((a.n + kBlock - 1) / kBlock);
   k_igr_prim<<<g, kBlock, 0, s>>>(a.n, u, a.prim, a.rinv);
   MFT_LAUNCH_CHECK();
   k_igr_rhs<<<g, kBlock, 0, s>>>(a);
   MFT_LAUNCH_CHECK();
+  if (a.staged) return launch_igr_staged(a, s);
   for (int it = 0; it < a.maxiter; ++it) {
     const double* uo = (it & 1) ? a.u1 : a.u0;
     double* un = (it & 1) ? a.u0 : a.u1;

@@ -498,17 +498,18 @@ struct IgrArgs {
   const double* wy;
   double alpha;
   int maxiter;
-  const float4* wxydw;  // double-word form: D_x, D_y as chunks on the forward layout, or null
-  double* prim;         // n x 3 (rho, v1, v2); double-word form: n x 4, two chunks per node
+  int staged;           // every row group has a neighbour list: the staged kernels
+  unsigned update_blocks;  // their update's grid, at most
+  double* prim;         // n x 3 (rho, v1, v2)
   double* rinv;         // n
   double* x;            // n: sigma
   double* r;            // n
   double* u0;           // n: CG directions, alternating
   double* u1;
   double* c;            // n
-  double* t;            // n x 2 (double-word form: one chunk per node)
+  double* t;            // n x 2
   double* add;          // n x 2 output: -(Dx sigma), -(Dy sigma)
-  double* partial;      // one double per block
+  double* partial;      // one double per block; staged: per group, and update_blocks more
   unsigned* counter;
   IgrScalars* sc;
 };
