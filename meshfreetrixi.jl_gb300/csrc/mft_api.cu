@@ -582,7 +582,7 @@ void ensure_work(mft_ctx* c) {
     c->tdw.alloc((size_t)n * 2 * V);
     c->qdw.alloc(nv);
   }
-  if (use_dw3(c)) c->Fdw.alloc((size_t)n * 14);  // a node's flux record, seven chunks
+  if (use_dw3(c)) c->Fdw.alloc((size_t)n * 12);  // a node's flux record, six chunks
   if (c->precision == MFT_PREC_FP32) {
     for (auto* b : {&c->U32[0], &c->U32[1], &c->U32[2], &c->U32[3]}) b->alloc(nv);
     c->du_p32.alloc(nv);
@@ -1047,7 +1047,9 @@ void eval_rhs(mft_ctx* c, double* us, float* us32, double t, const Epilogue& ep_
       }
       NvtxRange rng("calc fluxes");
       ProfScope ps(c, MFT_K_FWD);
-      launch_fwd3_dw(fa, s, !c->prof_on);  // profiling puts events between the two
+      // as its dependent where every group is staged (k_fwd3_dw), and not while profiling, which
+      // puts events between the two
+      launch_fwd3_dw(fa, s, !c->prof_on && c->fwd.halo_staged == c->fwd.halo_groups);
       return;
     }
     if (c->eq == MFT_EQ_EULER3D) {

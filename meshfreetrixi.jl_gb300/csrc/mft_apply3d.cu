@@ -21,7 +21,7 @@ namespace {
 
 using namespace dev;
 
-constexpr int kRec3 = 7;  // chunks of a node's double-word flux record
+constexpr int kRec3 = 6;  // chunks of a node's double-word flux record
 
 inline unsigned grid_for(int64_t n, int block) { return (unsigned)((n + block - 1) / block); }
 
@@ -95,11 +95,11 @@ __global__ void __launch_bounds__(kBlock) k_fwd3_f64(FwdArgs a) {
 // Double-word form: the state split into pairs and the flux formed in double-word
 // arithmetic (one reciprocal of rho refined by a Newton step).  The momentum flux is
 // symmetric, so the 15 flux components hold 12 distinct values, each formed once and stored
-// as the chunks of two that the gather multiplies (dw::chunk; xy = m1 m2 / rho and so on,
-// xx = m1 m1 / rho + p, ex = (E + p) v1):
-//   F[i] = (m1, ex), (m2, ey), (m3, ez), (xx, xy), (xy, yy), (xz, yz), (zz, zz)
-// (112 bytes), and F_x = (m1, xx, xy, xz, ex), F_y = (m2, xy, yy, yz, ey), F_z = (m3, xz, yz,
-// zz, ez).  The state is split on the integer pipe.
+// once, in chunks of two (dw::chunk; xy = m1 m2 / rho and so on, xx = m1 m1 / rho + p,
+// ex = (E + p) v1):
+//   F[i] = (m1, ex), (m2, ey), (m3, ez), (xx, xy), (yy, zz), (xz, yz)
+// (96 bytes, three sectors), and F_x = (m1, xx, xy, xz, ex), F_y = (m2, xy, yy, yz, ey),
+// F_z = (m3, xz, yz, zz, ez).  The state is split on the integer pipe.
 __global__ void k_prep_euler3d_dw(int64_t n, float2 gm1, const double* __restrict__ u,
                                   float4* __restrict__ F) {
   pdl_trigger();  // the gather may be launched: it waits for this kernel before it reads F
@@ -122,9 +122,8 @@ __global__ void k_prep_euler3d_dw(int64_t n, float2 gm1, const double* __restric
   Fi[1] = dw::chunk(m[1], ey);
   Fi[2] = dw::chunk(m[2], ez);
   Fi[3] = dw::chunk(xx, xy);
-  Fi[4] = dw::chunk(xy, yy);
+  Fi[4] = dw::chunk(yy, zz);
   Fi[5] = dw::chunk(xz, yz);
-  Fi[6] = dw::chunk(zz, zz);
 }
 
 // Running sums of the 3D gather: (mass, energy), (momentum 1, 2), and momentum 3 in three
@@ -143,24 +142,27 @@ static __device__ __forceinline__ void accum3(Sums3& s, float4 wxy, float2 wz, c
   dw::fma_acc2(s.f12, x, dw::pair2(q[3]));
   dw::fma_acc2(s.f3, dw::pair2(wxy), xzyz);
   dw::fma_acc2(s.f04, y, dw::pair2(q[1]));
-  dw::fma_acc2(s.f12, y, dw::pair2(q[4]));
-  dw::fma_acc(s.f3z, wz, dw::chunk_a(q[6]));
+  dw::fma_acc2(s.f12, y, dw::pair2(dw::chunk_b(q[3]), dw::chunk_a(q[4])));
+  dw::fma_acc(s.f3z, wz, dw::chunk_b(q[4]));
   dw::fma_acc2(s.f04, z, dw::pair2(q[2]));
   dw::fma_acc2(s.f12, z, xzyz);
 }
 
 // du_i = -sum_j (Dx_ij F_x + Dy_ij F_y + Dz_ij F_z)(node j) as compensated sums of
 // double-word products (mft_dw.cuh), the stage epilogue in FP64.  Per stencil entry: three
-// weight pairs and the neighbour's 112-byte flux record.  One block per row group
-// (ell.halo_rows rows) first stages the group's neighbour records in shared memory (seven
+// weight pairs and the neighbour's 96-byte flux record.  One block per row group
+// (ell.halo_rows rows) first stages the group's neighbour records in shared memory (six
 // 16-byte chunks each, mft_halo.cuh) and reads them from there; a group without a list
 // gathers directly.  Both read the same records in the same order: the same sums.
 // Bound by latency and issue of the packed FP32 products; the row's first weights are requested
 // before the staging, whose wait then covers theirs: 262k nodes 100 us -> 92.5 between events.
-// They are also requested before the flux kernel has ended (pdl_wait stands before the first
-// read of its records, and of anything else that is not constant): rhs! 133.1 -> 129.9 us.
-// The records are written while this grid is resident, so no read of them may take the
-// read-only path (__ldg): asynchronous copies or __ldcg.
+// Where every group is staged they are also requested before the flux kernel has ended (pdl_wait
+// stands before the first read of its records, and of anything else that is not constant):
+// rhs! 133.1 -> 129.9 us.  Direct reads take the read-only path through L1, which the records may
+// only do once they are complete, so a cloud with an unstaged group gets a plain launch (past L1
+// and as a dependent, 64^3 nodes: 378 us against 253 with 60 entries, 1721 of 2048 groups staged).
+// With xy, yy and zz in chunks of their own as they are multiplied (112 bytes, no moves) rhs! took
+// 133 us against 125, 157 / 141 with 35 entries, 253 / 215 with 60, 208 / 191 with none staged.
 __global__ void __launch_bounds__(kHaloRows, 2) k_fwd3_dw(FwdArgs a) {
   const int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   const float4* F4 = reinterpret_cast<const float4*>(a.Fdw);
@@ -207,7 +209,7 @@ __global__ void __launch_bounds__(kHaloRows, 2) k_fwd3_dw(FwdArgs a) {
       const float2 wz = __ldg(a.wzdw + p);
       float4 q[kRec3];
 #pragma unroll
-      for (int k = 0; k < kRec3; ++k) q[k] = __ldcg(F4 + c * kRec3 + k);
+      for (int k = 0; k < kRec3; ++k) q[k] = __ldg(F4 + c * kRec3 + k);
       accum3(f, wxy, wz, q);
     }
   }
@@ -239,7 +241,7 @@ void launch_fwd3_dw(const FwdArgs& a, cudaStream_t s, bool pdl) {
               MFT_ERR_STATE, "double-word 3D gather: arguments not set");
   MFT_REQUIRE(a.ell.halo_off && a.ell.halo_rows > 0, MFT_ERR_STATE,
               "double-word 3D gather: row groups not built");
-  // one block per row group, seven chunks of the longest list in dynamic shared memory
+  // one block per row group, six chunks of the longest list in dynamic shared memory
   // (above 48 KB a per-kernel opt-in, made once per device)
   const size_t smem = (size_t)kRec3 * a.ell.halo_stride * sizeof(float4);
   if (smem > 48 * 1024) {

@@ -342,11 +342,12 @@ void launch_fwd_f64(const FwdArgs& a, cudaStream_t s);
 // advection with the flux a_d u formed at the neighbour).
 void launch_flux_euler3d(int64_t n, double gamma, const double* u, double* F, cudaStream_t s);
 void launch_fwd3(const FwdArgs& a, cudaStream_t s);
-// The same for 3D Euler in double-word arithmetic: flux records (n x 14 float2, seven
+// The same for 3D Euler in double-word arithmetic: flux records (n x 12 float2, six
 // chunks) and the gather over the weights a.wxydw, a.wzdw.
 void launch_prep_euler3d_dw(int64_t n, double gamma, const double* u, float2* F,
                             cudaStream_t s);
-// pdl: the launch before in the stream is launch_prep_euler3d_dw (nothing between)
+// pdl: the launch before in the stream is launch_prep_euler3d_dw (nothing between), and every row
+// group has a neighbour list
 void launch_fwd3_dw(const FwdArgs& a, cudaStream_t s, bool pdl);
 // Double-word forms (mft_apply_dw.cu): per-node flux and state pairs, forward gather,
 // transpose gather.

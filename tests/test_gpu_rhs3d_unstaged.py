@@ -1,9 +1,9 @@
-"""The 3D gather launched beside the flux kernel it depends on, where row groups have no
-neighbour list and read the flux records from global memory: scattered node numbers kept as the
-layout order (no group staged, or half of them).  The same bits as with the gather launched
-after the flux kernel (profiling on, events between the two), for states that change from call
-to call; and the bits of the staged gather on the same cloud in Morton order (entries in structure
-order, so that every row forms the same sum in the same order)."""
+"""The 3D gather where row groups have no neighbour list and read the flux records from global
+memory, which the flux kernel before it must have completed: scattered node numbers kept as the
+layout order (no group staged, or half of them).  The same bits with the launches back to back and
+with events between them (profiling), for states that change from call to call; and the bits of
+the staged gather on the same cloud in Morton order (entries in structure order, so that every row
+forms the same sum in the same order)."""
 import numpy as np
 import pytest
 
