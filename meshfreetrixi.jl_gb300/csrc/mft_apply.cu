@@ -343,19 +343,10 @@ __device__ double block_sum_lanes(const double* v) {
   return r;
 }
 
-// |x| as a bit pattern: the sign bit cleared (fabs, without an FP64 instruction)
 typedef unsigned long long u64;
-constexpr u64 kAbsMask = 0x7FFFFFFFFFFFFFFFull;
-__device__ __forceinline__ u64 abs_key(double x) { return (u64)__double_as_longlong(x) & kAbsMask; }
-// The pattern of x as an unsigned integer that orders like the value (NaN beyond the
-// infinities on its sign's side), and back.
-__device__ __forceinline__ u64 order_key(double x) {
-  const u64 b = (u64)__double_as_longlong(x);
-  return b ^ ((b >> 63) ? ~0ull : 1ull << 63);
-}
-__device__ __forceinline__ double order_value(u64 k) {
-  return __longlong_as_double((long long)(k ^ ((k >> 63) ? 1ull << 63 : ~0ull)));
-}
+// |x| as a bit pattern: the sign bit cleared (fabs, without an FP64 instruction)
+__device__ __forceinline__ u64 abs_key(double x) { return fpbits::abs_bits((u64)__double_as_longlong(x)); }
+__device__ __forceinline__ u64 order_key(double x) { return fpbits::order_bits((u64)__double_as_longlong(x)); }
 __device__ __forceinline__ u64 warp_max_u64(u64 k) {
   const unsigned hi = (unsigned)(k >> 32), mh = __reduce_max_sync(kFull, hi);
   return ((u64)mh << 32) | __reduce_max_sync(kFull, hi == mh ? (unsigned)k : 0u);
@@ -372,12 +363,12 @@ __device__ __forceinline__ u64 block_max_u64(u64 k) {
   __syncthreads();
   return k;
 }
-// The first component's part of a lexicographic maximum of |u - mean| over nodes whose first
-// component lies in [lo, hi]: u - m rounds monotonically, so the largest |u - m| is that of an
-// end.
+// The first component's part of a lexicographic maximum of |u - mean| over a block's nodes, whose
+// first component lies between its extremes (order keys); 0 for a block without nodes.
 __device__ __forceinline__ u64 extreme_key(u64 lo, u64 hi, double m) {
-  const u64 a = abs_key(dsub(order_value(lo), m)), b = abs_key(dsub(order_value(hi), m));
-  return a > b ? a : b;
+  return fpbits::extreme_abs(lo, hi, [&](uint64_t b) {
+    return (uint64_t)__double_as_longlong(dsub(__longlong_as_double((long long)b), m));
+  });
 }
 
 // Sum of u per variable; the last block to finish reduces the block partials in a fixed
@@ -392,7 +383,7 @@ __global__ void __launch_bounds__(kBlock) k_mean(int64_t n, const double* __rest
                                                  u64* top) {
   pdl_trigger();
   double acc[V];
-  u64 nlo = 0, hi = 0;  // the complement of the lowest order key, and the highest
+  u64 nlo = ~fpbits::kLowest, hi = 0;  // the complement of the lowest order key, and the highest
 #pragma unroll
   for (int k = 0; k < V; ++k) acc[k] = 0.0;
   // unrolled so that four nodes' loads are in flight together; the additions keep the

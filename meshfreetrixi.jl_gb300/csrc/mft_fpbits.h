@@ -88,6 +88,25 @@ MFT_FPBITS_FN bool split_words(uint32_t hi, uint32_t lo, uint32_t* h, int32_t* r
   return true;
 }
 
+// ---------------------------------------------------------------- order keys
+// The IEEE pattern b of a double as an unsigned integer that orders like the value (NaN beyond
+// the infinities on its sign's side), and back; |x| as a pattern.
+MFT_FPBITS_FN uint64_t order_bits(uint64_t b) { return b ^ ((b >> 63) ? ~0ull : 1ull << 63); }
+MFT_FPBITS_FN uint64_t order_back(uint64_t k) { return k ^ ((k >> 63) ? 1ull << 63 : ~0ull); }
+MFT_FPBITS_FN uint64_t abs_bits(uint64_t b) { return b & 0x7FFFFFFFFFFFFFFFull; }
+
+// The lowest and highest order keys of a set start as kLowest, 0 (lo > hi: an empty set).
+// Largest pattern of |x - m| over a set whose values lie between its extremes: the rounded
+// difference is monotonic in x, so that of an end; 0, the smallest, for an empty set.
+// diff(b): the pattern of (value of pattern b) - m.
+constexpr uint64_t kLowest = ~0ull;
+template <typename Diff>
+MFT_FPBITS_FN uint64_t extreme_abs(uint64_t lo, uint64_t hi, Diff diff) {
+  if (lo > hi) return 0;
+  const uint64_t a = abs_bits(diff(order_back(lo))), b = abs_bits(diff(order_back(hi)));
+  return a > b ? a : b;
+}
+
 }  // namespace fpbits
 
 #if defined(__CUDACC__)
