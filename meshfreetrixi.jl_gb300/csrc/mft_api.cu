@@ -1086,7 +1086,7 @@ void eval_rhs(mft_ctx* c, double* us, float* us32, double t, const Epilogue& ep_
     na.partial = c->red_partial.p;
     na.counter = c->red_counter.p;
     na.nblocks = c->red_blocks;
-    if (c->nseg > 0 || n <= kNormClusterMax) {
+    if (c->nseg > 0 || n <= (f32 ? kNormClusterMaxF32 : kNormClusterMax)) {
       if (!c->prof_on) {
         launch_norms_cluster(na, 3, st);
       } else {

@@ -391,6 +391,11 @@ void launch_norm_lexmax(const NormArgs& a, bool pdl, cudaStream_t s);
 // two grid reductions cost a launch and two last-block tails; one rhs! with the grid reductions /
 // the cluster: 4,096 nodes 78 / 51 us, 32,761: 76 / 71, 65,536: 97 / 86, 131,044: 122 / 146.
 constexpr int64_t kNormClusterMax = 65536;
+// In the FP32 form they run beside a gather that is shorter than one cluster's pass over many
+// nodes; a stage of SSP-RK3 with the grid reductions / the cluster: 16,384 nodes 28.0 / 25.0 us,
+// 22,500: 30.1 / 29.0, 32,761: 30.7 / 32.7, 40,000: 31.4 / 34.4, 65,536: 35.0 / 43.8.  (The FP64
+// forms beside longer gathers: 65,536 nodes 142 / 141, 40,000 with the double-word sums 61 / 62.)
+constexpr int64_t kNormClusterMaxF32 = 24576;
 void launch_norms_cluster(const NormArgs& a, int phases, cudaStream_t s);
 
 void launch_eps(const EpsArgs& a, cudaStream_t s);
