@@ -684,6 +684,7 @@ void ensure_device_ops(mft_ctx* c) {
                           chunked ? k : -1, s);
   }
   MFT_CUDA(cudaStreamSynchronize(s));
+  c->d_st_ci.release();  // 4 k bytes per node; weights formed after this upload st_ci
   c->dev_dirty = false;
   for (int &k : c->tuned_fwd) k = -1;
   for (int &k : c->tuned_rev) k = -1;
@@ -1553,6 +1554,7 @@ mft_status mft_set_points(mft_ctx* c, int dim, int64_t n, const double* xyz, con
         MFT_REQUIRE(period[d] > 0.0, MFT_ERR_ARG, "period lengths must be positive");
     c->d_xyz.upload(c->xyz, c->stream);
     c->have_stencils = false;
+    c->d_st_ci.release();
     c->have_pattern = false;
     for (int k = 0; k < kSlots; ++k) c->have_val[k] = false;
     c->dev_dirty = true;
@@ -1689,6 +1691,7 @@ mft_status mft_load_csc(mft_ctx* c, int op, int comp, int64_t n, const int64_t* 
       finish_pattern(c);
       c->st2csr.clear();
       c->have_stencils = false;
+      c->d_st_ci.release();
     }
     const int slot = op == MFT_OP_GRAD ? comp : (op == MFT_OP_LAP ? kSlotLap : kSlotHv);
     c->val[slot].resize(nnz);

@@ -33,7 +33,9 @@ struct mft_ctx {
   // stencils in caller order (centre first)
   std::vector<int64_t> st_rp;
   mft::HostVec<int32_t> st_ci;
-  mft::DBuf<int32_t> d_st_ci;  // the same on the device after mft_knn (empty: upload st_ci)
+  // the same on the device, from mft_knn to the first evaluation or the next cloud or stencils
+  // (empty: upload st_ci)
+  mft::DBuf<int32_t> d_st_ci;
   bool have_stencils = false;
 
   // operator pattern: CSR rows with ascending columns, its CSC view, and maps
