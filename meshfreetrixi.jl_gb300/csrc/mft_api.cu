@@ -1591,9 +1591,6 @@ mft_status mft_knn(mft_ctx* c, int k, int32_t* out_idx, double* out_dist, double
     set_device(c);
     double dmin = 0, davg = 0;
     knn_device(c, k, out_idx, out_dist, &dmin, &davg);
-    c->st_rp.resize(c->n + 1);
-    for (int64_t i = 0; i <= c->n; ++i) c->st_rp[i] = i * k;
-    c->have_stencils = true;
     pattern_from_stencils(c);
     if (out_dx_min) *out_dx_min = dmin;
     if (out_dx_avg) *out_dx_avg = davg;
@@ -1629,11 +1626,11 @@ mft_status mft_weights(mft_ctx* c, int op, int rbf_pow, int polydeg, int deriv_o
       for (int d = 0; d < D; ++d) {
         c->val[d].resize(nnz);
         v[d] = c->val[d].data();
-        c->have_val[d] = true;
       }
 #pragma omp parallel for schedule(static)
       for (int64_t e = 0; e < nnz; ++e)
         for (int d = 0; d < D; ++d) v[d][to[e]] = w[e * D + d];
+      for (int d = 0; d < D; ++d) c->have_val[d] = true;
     } else {
       const int slot = op == MFT_OP_LAP ? kSlotLap : kSlotHv;
       c->val[slot].resize(nnz);

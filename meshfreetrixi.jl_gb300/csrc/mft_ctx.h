@@ -230,9 +230,9 @@ void pattern_from_stencils(mft_ctx* c);
 // Reverse CSC view + ELL/maps rebuild flags after the CSR pattern is set.
 void finish_pattern(mft_ctx* c);
 // KNN and weights (mft_knn.cu, mft_weights.cu)
-// knn_device: the stencils into c->st_ci (kept on the device in c->d_st_ci) and, where given,
-// out_idx; the distances into dist (n k) where given.  weights_device: st_ci.size() dim values
-// into w.
+// knn_device: the stencils into c->st_ci and c->st_rp (kept on the device in c->d_st_ci) and, where
+// given, out_idx; a call that fails leaves the context's as they were.  The distances into dist
+// (n k) where given.  weights_device: st_ci.size() dim values into w.
 void knn_device(mft_ctx* c, int k, int32_t* out_idx, double* dist, double* dx_min, double* dx_avg);
 void weights_device(mft_ctx* c, int rbf_pow, int polydeg, int deriv_order, double* w,
                     double* max_resid);

@@ -414,10 +414,11 @@ void knn_device(mft_ctx* c, int k, int32_t* out_idx, double* dist, double* dx_mi
   }
   MFT_CUDA(cudaStreamSynchronize(s));
   MFT_REQUIRE(err == 0, MFT_ERR_ARG, "KNN search could not collect k neighbours");
-  std::swap(c->d_st_ci.p, d_idx.p);
-  std::swap(c->d_st_ci.n, d_idx.n);
-  c->st_ci.resize((size_t)n * k);
-  copy_out(c, c->st_ci.data(), c->d_st_ci.p, c->st_ci.size() * sizeof(int32_t), out_idx);
+  // the context's stencils are replaced at the end, where nothing can fail any more
+  HostVec<int32_t> ci((size_t)n * k);
+  std::vector<int64_t> rp(n + 1);
+  for (int64_t i = 0; i <= n; ++i) rp[i] = i * k;
+  copy_out(c, ci.data(), d_idx.p, ci.size() * sizeof(int32_t), out_idx);
   if (dist) {
     if (k >= 2) copy_out(c, dist, d_d2.p, (size_t)n * k * sizeof(double));
     else std::fill(dist, dist + n, 0.0);  // the node itself
@@ -435,6 +436,11 @@ void knn_device(mft_ctx* c, int k, int32_t* out_idx, double* dist, double* dx_mi
     if (dx_min) *dx_min = NAN;
     if (dx_avg) *dx_avg = NAN;
   }
+  c->st_ci.swap(ci);
+  c->st_rp.swap(rp);
+  std::swap(c->d_st_ci.p, d_idx.p);
+  std::swap(c->d_st_ci.n, d_idx.n);
+  c->have_stencils = true;
 }
 
 }  // namespace mft
