@@ -289,7 +289,7 @@ mft_status mft_set_option(mft_ctx* ctx, int option, int value);
 /* Reads an option; MFT_OPT_TUNED_FWD / MFT_OPT_TUNED_REV return the mapping the
  * autotuner chose for the most recent forward / transpose gather launch: FP32 form
  * 0 = one node per thread, 4 or 8 = staged with that many slots per bulk copy; FP64
- * form with double-word gathers: the kernel variant 0..5; -1 = not tuned yet. */
+ * form with double-word gathers: the kernel variant 0..12; -1 = not tuned yet. */
 mft_status mft_get_option(mft_ctx* ctx, int option, int* value);
 
 /* Self-test of the bounded-wait error path (no fault involved): one warp waits on a

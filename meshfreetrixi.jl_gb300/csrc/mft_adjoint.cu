@@ -195,7 +195,7 @@ __global__ void k_lam_pairs(int64_t n, const double* __restrict__ lam, BcDev bc,
 // run on the integer pipe, and where every group is staged the kernel that writes them for every
 // node (k_lam_pairs) is not launched (one launch per stage, 65,536 nodes).  A group without a list
 // reads that kernel's chunks, one 32-byte load per entry: forming them per entry took 169 us
-// against 140 at 262,144 scattered nodes, none staged.  With the
+// against 125 at 262,144 scattered nodes, none staged.  With the
 // streamed loads in groups of kAdjGroup ahead the gather and that kernel took 26.4 us between
 // events against 29.2 (groups of 2 / 3 / 4 / 5: 27.4 / 27.0 / 26.3 / 27.2); without that kernel and
 // with the first entries requested before the staging 23.9.

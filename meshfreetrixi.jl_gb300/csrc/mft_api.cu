@@ -849,8 +849,8 @@ static int rev_choice(mft_ctx* c, const RevArgs& a) {
   return c->tuned_rev[key];
 }
 
-// The double-word gathers have four kernel variants (plain or software-pipelined loop,
-// with or without a register cap); with MFT_OPT_DW_VARIANT < 0 (default) the first
+// The double-word gathers have kDwVariants kernel variants (direct or staged neighbours, loop
+// forms, register caps, prefetch and cache hints); with MFT_OPT_DW_VARIANT < 0 (default) the first
 // launch of each configuration outside a graph capture times them on the live inputs and
 // keeps the fastest until the operators change.
 static int dw_fwd_choice(mft_ctx* c, const FwdArgs& a) {
@@ -913,10 +913,7 @@ void launch_rev(mft_ctx* c, const RevArgs& a) {
   }
 }
 
-// Device error word set by kernels with bounded waits; read at synchronisation points.
-// Synchronises the stream and reads the word: the word's copy into pinned memory is
-// queued behind the work, so one synchronisation covers both.
-// Pinned host copy of the error word, mapped for the device.
+// Pinned host copy of the device error word, mapped for the device.
 static int* host_error_word(mft_ctx* c) {
   if (!c->h_kerr) {
     MFT_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&c->h_kerr), sizeof(int), cudaHostAllocMapped));
@@ -924,7 +921,10 @@ static int* host_error_word(mft_ctx* c) {
   }
   return c->h_kerr;
 }
-// brought: the call's last kernel has written the word (launch_soa_from_aos).
+// Device error word set by kernels with bounded waits and by non-finite outputs; read at
+// synchronisation points.  Synchronises the stream and reads the word: its copy into pinned memory
+// is queued behind the work, so one synchronisation covers both.  brought: the call's last kernel
+// has written the word there already (launch_soa_from_aos).
 static void check_kernel_errors(mft_ctx* c, bool brought = false) {
   if (!c->kerr.p) {
     MFT_CUDA(cudaStreamSynchronize(c->stream));
@@ -1014,7 +1014,7 @@ void eval_rhs(mft_ctx* c, double* us, float* us32, double t, const Epilogue& ep_
   }
   if (c->dim == 3) {
     // 3D clouds: the plain flux divergence (calc_fluxes! over D_x, D_y, D_z) with the
-    // strong BCs and the stage epilogue, in FP64 fused multiply-adds
+    // strong BCs and the stage epilogue, in double-word sums or FP64 fused multiply-adds
     MFT_REQUIRE(!f32, MFT_ERR_UNSUPPORTED, "3D point clouds: the FP64 form only");
     MFT_REQUIRE(iv < 0 && ih < 0 && ig < 0, MFT_ERR_UNSUPPORTED,
                 "3D point clouds: no viscosity, hyperviscosity or IGR source (the "
@@ -1803,7 +1803,7 @@ mft_status mft_set_option(mft_ctx* c, int option, int value) {
       for (int& k : c->tuned_rev) k = -1;
     } else if (option == MFT_OPT_DW_VARIANT) {
       MFT_REQUIRE(value >= -1 && value < kDwVariants, MFT_ERR_ARG,
-                  "double-word gather variant: -1 (tuned) or 0..5");
+                  "double-word gather variant: -1 (tuned) or 0..12");
       c->dw_variant = value;
       c->fsal_valid = false;
     } else if (option == MFT_OPT_HALO_ROWS) {

@@ -57,9 +57,9 @@ static __device__ __forceinline__ void prefetch_chunk(const SliceArrays& sa, int
 // operation is accurate to about 2 u^2 of its operands, u = 2^-24), as the records the
 // forward gather reads, in chunks of two values (dw::chunk): U = (rho, m1), (m2, E) and
 // F = (fx1, f12), (f12, fy2), (fx3, fy3), (m1, m2), with f12 = m1 m2 / rho the x flux of m2
-// and the y flux of m1; the mass fluxes are m1 and m2.  gm1 = gamma - 1 as a pair.  The only
-// FP64 operations are the four splits of the state.  Shared by the flux kernel and the staged
-// gathers that form the records while staging, so both give the same bits.
+// and the y flux of m1; the mass fluxes are m1 and m2.  gm1 = gamma - 1 as a pair.  The state is
+// split on the integer pipe.  Shared by the flux kernel and the staged gathers that form the
+// records while staging, so both give the same bits.
 static __device__ __forceinline__ void euler_records(double2 a, double2 b, float2 gm1,
                                                      float4* F, float4* U) {
   const float2 rho = dw::split(a.x), m1 = dw::split(a.y), m2 = dw::split(b.x);
@@ -248,8 +248,9 @@ static __device__ __forceinline__ void fwd_accum(const FwdEntry& e, FwdSums& s) 
 
 // Forward gather (Euler), one node per thread over the sliced ELL: the flux divergence
 // -sum_j (Dx F_x + Dy F_y), t = (Dx u, Dy u) (WT), q = lap u (WQ) or the Flyer term
-// H u (FLY), as in k_fwd_euler_f64.  Per stencil entry: a 64-byte flux record and a
-// 32-byte state record (both one or two 256-bit loads), 8-byte weights.
+// H u (FLY), as in k_fwd_euler_f64.  Per stencil entry: the weights' 16-byte chunk (and 8 bytes
+// more for q or H u), and of the neighbour three flux chunks and the state's two, or four flux
+// chunks where the state is not needed (read directly: 256-bit loads).
 // PIPE = 0: one entry per loop iteration; PIPE = 2: two (the compiler overlaps their
 // loads); PIPE = 1: software pipeline -- the column index is loaded two entries ahead and
 // the weights and records one entry ahead, so that the gathers of entry j + 1 are in flight while entry j is

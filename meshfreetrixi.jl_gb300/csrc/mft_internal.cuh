@@ -38,8 +38,11 @@ struct Error : std::runtime_error {
 // while the previous kernel in its stream still runs, once every block of that kernel has
 // executed pdl_trigger() (or exited); before reading anything that kernel writes it must
 // execute pdl_wait(), which returns when that kernel has completed and its writes are
-// visible (at once for a grid launched without the attribute).  Everything earlier in the
-// stream has completed before the previous kernel started, as with plain launches.
+// visible (at once for a grid launched without the attribute).  Where the previous kernel was a
+// plain launch, everything earlier in the stream had completed before it started; in a chain of
+// dependents that holds only because each of them waits before it ends.  Memory that the previous
+// kernel writes may not be read through the read-only path (__ldg, const __restrict__): that asks
+// that nobody writes it while the grid is resident.
 __device__ __forceinline__ void pdl_trigger() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
